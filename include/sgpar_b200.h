@@ -175,9 +175,11 @@ typedef struct {
     uint32_t cluster_max_log2;  /* power-iteration levels above one block's shared memory and of at
                                    most 2^k cost units (entries + 8 per vertex) run on a cluster of
                                    blocks (one cluster barrier per iteration, several levels at
-                                   once); larger ones on the whole GPU.  0 = the default: 17 for
-                                   single partitions, 23 for sgp_b200_partition_batch, whose levels
-                                   of many graphs then share the GPU.  Equal values give equal bits. */
+                                   once); larger ones on the whole GPU.  0 = the default: 23 for
+                                   sgp_b200_partition_batch, whose levels of many graphs then share
+                                   the GPU; for single partitions none of the FP64 levels, which run
+                                   on the whole GPU, and 17 for those of the mixed-precision and the
+                                   normalized variants.  Equal values give equal bits. */
     uint32_t cluster_blocks;    /* blocks per cluster of that kernel: 8 or 2.  0 = the default: 8 for
                                    single partitions (each level's latency), 2 for
                                    sgp_b200_partition_batch (twice as many hierarchies iterate at

@@ -297,6 +297,7 @@ static int eigen_finish(Context &C, std::vector<Level> &levels, const PowerIterO
         // relabelled copy of it would not pay for itself
         PowerIterOpts ol = o;
         ol.allow_relabel = o.allow_relabel && l > 0;
+        ol.probe = l == 0;
         SGPB_TRY(power_iter_level(C, lv, xin, vc, xo, ol, &r, l == 0));
         lv.pi_iters = r.niter;
         lv.pi_ms = r.kernel_ms;
@@ -353,11 +354,11 @@ static int partition_begin(Context &C, const Level &L0, const sgp_b200_options_t
     S->po.iter_cap = opt->iter_cap;
     S->po.mixed = opt->mixed;
     S->po.normlap = opt->refine_alg == 1;
-    // the cluster kernel's share of the levels: up to 2^17 cost units for a
-    // single partition (latency), 2^23 in a batch (many levels at once)
+    // the cluster kernel's share of the levels: up to 2^23 cost units in a
+    // batch (many levels at once); the levels' own rule in a single partition
     const uint32_t lg = opt->cluster_max_log2 ? (opt->cluster_max_log2 < 40 ? opt->cluster_max_log2 : 40u)
-                                              : (batch ? 23u : 17u);
-    S->po.mid_limit = 1ull << lg;
+                                              : (batch ? 23u : 0u);
+    S->po.mid_limit = lg ? 1ull << lg : 0ull;
     // blocks per cluster: 8 for a single partition, 2 in a batch
     if (opt->cluster_blocks != 0 && opt->cluster_blocks != 2 && opt->cluster_blocks != 8) {
         set_error("options.cluster_blocks must be 0, 2 or 8 (got %u)", opt->cluster_blocks);

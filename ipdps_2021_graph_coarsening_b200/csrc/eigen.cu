@@ -47,6 +47,7 @@
 
 #include "common.cuh"
 #include "internal.h"
+#include "pi_common.cuh"
 
 namespace sgpb {
 
@@ -81,7 +82,7 @@ struct PIArgs {
     double *partials;             // [2][gridDim][kNP]
     double tol;
     uint64_t iter_max;
-    double *res;                  // [0] niter [1] dot [2] gb [3] lambda [4] capped
+    double *res;                  // [0] niter [1] dot [2] gb [3] lambda [4] capped [6] the dot before the last
     const uint32_t *inv;          // relabelled copy: new id -> level vertex id (null: identity)
     uint32_t kcache;              // leading iterate entries: shared-memory copy, or the L1 hub prefix
     int cache_ok;                 // host: 2 shared-memory copy when it fits, 3 L1 hub prefix, 0 none
@@ -591,7 +592,6 @@ __device__ __forceinline__ void warp_stream(const uint32_t *__restrict__ rp, con
 // multicast.
 constexpr uint32_t kStageCh = kStagePad;
 constexpr int kStageU = 8;                       // entries per lane per trip (32 * 8 = kStageCh)
-constexpr uint32_t kStageWaitLimit = 1u << 22;   // bounded mbarrier polls before giving up
 template <typename W>
 struct StageCfg {
     static constexpr uint32_t R = sizeof(W) == 8 ? 2 : (sizeof(W) == 4 ? 3 : 4);   // ring slots per warp
@@ -599,37 +599,6 @@ struct StageCfg {
     static constexpr size_t warp_bytes = ((size_t)R * kStageCh * (4 + sizeof(W)) + 12 * R + 15) & ~(size_t)15;
 };
 
-__device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t *b) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(b)) : "memory");
-}
-__device__ __forceinline__ void mbar_fence_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *b, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(b)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_test(uint64_t *b, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_addr(b)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// bounded wait for the phase of the given parity to complete
-__device__ __forceinline__ bool mbar_wait(uint64_t *b, uint32_t parity) {
-    for (uint32_t k = 0; k < kStageWaitLimit; k++)
-        if (mbar_test(b, parity)) return true;
-    return false;
-}
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *b) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_addr(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_addr(b))
-                 : "memory");
-}
 // generic-proxy reads of a slot are ordered before the next bulk copy into it
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
@@ -931,23 +900,6 @@ __device__ __forceinline__ void panel_rows32(const uint32_t *__restrict__ offp, 
     }
     if (lane < gl) yacc[g + lane] = yprev + ysm[lane];
     __syncwarp();
-}
-
-// The next raw iterate value r_i of row i from u_i = (x_i - mu) / nu and
-// its row sum acc (plain: sum_j w_ij x_j; MX: sum_j w_ij (x_i - x_j)):
-// shifted Laplacian r = (gb - d) u + A u = gb u - L u, or the lazy random
-// walk r = u / 2 + (A u)_i / (2 d) of the normalized variant (r = u / 2 for
-// an isolated vertex).  All in FP64.
-template <bool MX>
-__device__ __forceinline__ double next_value(int normlap, double gb, double mu, double inv_nu, double ui, double acc,
-                                             double d) {
-    if constexpr (MX) {
-        const double lu = acc * inv_nu;   // (L u)_i; the mean cancels in the differences
-        return normlap ? (d > 0 ? ui - 0.5 * lu / d : 0.5 * ui) : gb * ui - lu;
-    } else {
-        const double au = (acc - mu * d) * inv_nu;   // (A u)_i
-        return normlap ? 0.5 * ui + (d > 0 ? 0.5 * au / d : 0.0) : (gb - d) * ui + au;
-    }
 }
 
 template <int CACHE, typename V>
@@ -1323,6 +1275,7 @@ __global__ void __launch_bounds__(kPIThreads, 2) k_power_iter(PIArgs a) {
                 a.res[3] = a.normlap ? 2.0 * (1.0 - S[2] / S[4]) : (gb * S[4] - S[2]) / S[4];
                 a.res[4] = niter >= a.iter_max ? 1.0 : 0.0;
                 a.res[5] = 0.0;
+                a.res[6] = last;
             }
             return;
         }
@@ -1526,12 +1479,6 @@ struct PIChainDesc {
     PIArgs a;
     int wbytes;   // 0, 4 or 8
 };
-
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
 
 // Work queue over chains (the host orders them largest first): each block
 // takes the next chain from a counter and runs its levels in order, so one
@@ -2206,7 +2153,7 @@ static int launch_pi(Context &C, PIArgs &a, uint32_t grid, int mode) {
 // levels, else the cooperative kernel (column panels when a layout is given).
 // mixed: FP32 edge-difference arithmetic (never with panels or small levels).
 static int run_pi(Context &C, const Level &L, PIArgs a, bool mixed, const PanelLayout *panels, double *res_d,
-                  double res_h[5], float *ms, uint32_t grid, int mode) {
+                  double res_h[7], float *ms, uint32_t grid, int mode) {
     a.res = res_d;
     a.P = 0;
     if (panels) {
@@ -2257,9 +2204,9 @@ static int run_pi(Context &C, const Level &L, PIArgs a, bool mixed, const PanelL
     cudaEventRecord(e1, C.stream);
     if (rc != SGP_B200_OK) { cudaEventDestroy(e0); cudaEventDestroy(e1); return rc; }
     SGPB_CUDA(cudaGetLastError());
-    SGPB_CUDA(cudaMemcpyAsync(C.h_pinned, res_d, 6 * sizeof(double), cudaMemcpyDeviceToHost, C.stream));
+    SGPB_CUDA(cudaMemcpyAsync(C.h_pinned, res_d, 7 * sizeof(double), cudaMemcpyDeviceToHost, C.stream));
     SGPB_CUDA(cudaStreamSynchronize(C.stream));
-    memcpy(res_h, C.h_pinned, 5 * sizeof(double));
+    memcpy(res_h, C.h_pinned, 7 * sizeof(double));
     if (!small && ((const double *)C.h_pinned)[5] != 0.0) {
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
@@ -2393,7 +2340,7 @@ static int autotune_level(Context &C, const Level &L, const PIArgs &a0, bool mix
         a.out = scratch;
         a.iter_max = kTuneIters;
         a.tol = -1.0;   // run exactly kTuneIters iterations
-        double rh[5];
+        double rh[7];
         float k = 0;
         SGPB_TRY(run_pi(C, L, a, mixed, nullptr, res_d, rh, &k, pi_grid(C, L.n, L.m, c.units), c.mode));
         *ms = k;
@@ -2431,6 +2378,12 @@ static int autotune_level(Context &C, const Level &L, const PIArgs &a0, bool mix
     return SGP_B200_OK;
 }
 
+// Iterations a level with o.probe takes before its row slices are laid out,
+// and the entries below which it is laid out at once.  R-MAT 22's input level
+// stops after two.
+constexpr uint64_t kProbeIters = 4;
+constexpr uint64_t kProbeMinM = 1ull << 20;
+
 int power_iter_level(Context &C, const Level &Lin, const double *x_in, const uint32_t *vcmap, double *x_out,
                      const PowerIterOpts &o, PowerIterResult *res, int want_residual) {
     const uint32_t n = Lin.n;
@@ -2461,6 +2414,16 @@ int power_iter_level(Context &C, const Level &Lin, const double *x_in, const uin
         ch.lev.push_back(cl);
         SGPB_TRY(power_iter_mid_chains(C, {&ch}, o));
         *res = ch.lev[0].res;
+        if (want_residual) SGPB_TRY(level_residual(C, Lin, x_out, o.normlap, res));
+        return SGP_B200_OK;
+    }
+    // FP64 levels run on row slices.  A level that may stop after a few
+    // iterations (o.probe) takes its first ones on the kernel below, which
+    // needs no layout, and goes on from their iterate only if it has to.
+    const bool slices = power_iter_slices_ok(Lin, o);
+    const bool probe = slices && o.probe && Lin.m >= kProbeMinM;
+    if (slices && !probe) {
+        SGPB_TRY(power_iter_slices(C, Lin, x_in, vcmap, x_out, o, iter_budget(n, o), 0, 0.0, res));
         if (want_residual) SGPB_TRY(level_residual(C, Lin, x_out, o.normlap, res));
         return SGP_B200_OK;
     }
@@ -2531,16 +2494,24 @@ int power_iter_level(Context &C, const Level &Lin, const double *x_in, const uin
     SGPB_TRY(setup_split(C, L, tune, a));
     a.out = x_out;
     const uint64_t imax = iter_budget(n, o);
-    a.iter_max = imax;
+    a.iter_max = probe && imax > kProbeIters ? kProbeIters : imax;
     a.tol = o.tol;
     double *res_d;
     SGPB_TRY(dalloc_t(C, &res_d, 8));
-    double rh[5];
+    double rh[7];
     float kms = 0;
     PanelLayout panels;
     if (want_panels) SGPB_TRY(build_panels(C, L, a.heavy_T, sizeof(double), &panels));
     SGPB_TRY(run_pi(C, L, a, mixed, want_panels ? &panels : nullptr, res_d, rh, &kms, pi_grid(C, n, L.m, tune.units),
                     tune.mode));
+    if (a.iter_max < imax && rh[4] != 0.0) {
+        // not converged: repeat the last iteration from the vector it began
+        // with, the dot product before it carried over
+        SGPB_TRY(power_iter_slices(C, Lin, x_out, nullptr, x_out, o, imax, kProbeIters - 1, rh[6], res));
+        res->kernel_ms += kms;
+        if (want_residual) SGPB_TRY(level_residual(C, Lin, x_out, o.normlap, res));
+        return SGP_B200_OK;
+    }
     const uint64_t total_iters = (uint64_t)rh[0];
     res->niter = total_iters;
     res->dot = rh[1];
@@ -2692,6 +2663,7 @@ bool power_iter_mid_ok(const Level &L, const PowerIterOpts &o) {
         if (atoi(e) == 0) return false;
     if (L.n == 0 || power_iter_small_ok(L, o)) return false;
     if (!(L.wbytes == 0 || L.wbytes == 4 || L.wbytes == 8)) return false;
+    if (!o.mid_limit && power_iter_slices_ok(L, o)) return false;
     return L.m + 8ull * L.n <= (o.mid_limit ? o.mid_limit : kMidCost);
 }
 

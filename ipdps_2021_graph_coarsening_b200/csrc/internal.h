@@ -165,7 +165,9 @@ struct PowerIterOpts {
     int mixed = 0;           // 1: FP32 edge-difference SpMV arithmetic, FP64 iterate and reductions
     int allow_relabel = 1;   // skewed levels may iterate on a hub-first relabelled copy
     int normlap = 0;         // refine_alg 1: normalized-Laplacian (lazy random walk) iteration
-    uint64_t mid_limit = 0;  // largest cost (m + 8n) of a level on the cluster kernel; 0 = 2^17
+    int probe = 0;           // 1: the level may stop after a few iterations (the finest one)
+    uint64_t mid_limit = 0;  // largest cost (m + 8n) of a level on the cluster kernel; 0 = the rule:
+                             // 2^17, and none of the levels that run on row slices
     int mid_blocks = 0;       // blocks per cluster of the cluster kernel (2 or 8); 0 = 8
 };
 struct PowerIterResult {
@@ -178,6 +180,16 @@ struct PowerIterResult {
 // initial vector; x_out: n doubles (may alias nothing).
 int power_iter_level(Context &C, const Level &L, const double *x_in, const uint32_t *vcmap,
                      double *x_out, const PowerIterOpts &o, PowerIterResult *res, int want_residual);
+// The same recurrence on row slices (slices.cu): FP64 levels of any size.
+// iter0 / dot0: iterations already done on the vector x_in and the dot
+// product before its last one (0 and 0 for a fresh start); their number counts
+// towards iter_max and the result's niter.
+bool power_iter_slices_ok(const Level &L, const PowerIterOpts &o);
+int power_iter_slices(Context &C, const Level &L, const double *x_in, const uint32_t *vcmap, double *x_out,
+                      const PowerIterOpts &o, uint64_t iter_max, uint64_t iter0, double dot0, PowerIterResult *res);
+// order of the vertices by descending degree class (eight classes an octave),
+// stable inside a class: perm (vertex -> new id) and inv
+int degree_order(Context &C, uint32_t n, const uint32_t *rp, uint32_t **perm, uint32_t **inv);
 // |L x - lambda x| / (bound on the spectrum) of a level's result into res->resid
 int level_residual(Context &C, const Level &L, const double *x, int normlap, PowerIterResult *res);
 // Small levels (one block, the level in shared memory).  A chain is the

@@ -16,24 +16,31 @@
 
 namespace sgpb {
 
-constexpr int kBuckets = 33;       // floor(log2(deg)) + 1 for deg >= 1, 0 for deg == 0
+// Degree classes: floor(log2(deg)) + 1 for deg >= 1 and 0 for deg == 0, each
+// cut into 2^SUB by the bits below the leading one.
+template <int SUB>
+constexpr int kBuckets = 33 << SUB;
 constexpr int kPermTile = 1024;    // rows per block of the stable scatter
 
+template <int SUB>
 __device__ __forceinline__ uint32_t deg_key(uint32_t deg) {
     // key 0 = highest degree class; ascending key = descending degree
     const uint32_t b = deg ? 32u - __clz(deg) : 0u;   // 1..32, 0 for empty
-    return (uint32_t)(kBuckets - 1) - b;
+    uint32_t sub = 0;
+    if (SUB > 0 && deg) sub = (b > SUB ? deg >> (b - 1 - SUB) : deg << (SUB + 1 - b)) & ((1u << SUB) - 1u);
+    return (uint32_t)(kBuckets<SUB> - 1) - ((b << SUB) | sub);
 }
 
+template <int SUB>
 __global__ void k_bucket_count(uint32_t n, const uint32_t *rp, uint32_t nb, uint32_t *cnt) {
-    __shared__ uint32_t c[kBuckets];
-    for (int k = threadIdx.x; k < kBuckets; k += blockDim.x) c[k] = 0;
+    __shared__ uint32_t c[kBuckets<SUB>];
+    for (int k = threadIdx.x; k < kBuckets<SUB>; k += blockDim.x) c[k] = 0;
     __syncthreads();
     const uint64_t t0 = (uint64_t)blockIdx.x * kPermTile;
     for (uint64_t i = t0 + threadIdx.x; i < t0 + kPermTile && i < n; i += blockDim.x)
-        atomicAdd(&c[deg_key(rp[i + 1] - rp[i])], 1u);
+        atomicAdd(&c[deg_key<SUB>(rp[i + 1] - rp[i])], 1u);
     __syncthreads();
-    for (int k = threadIdx.x; k < kBuckets; k += blockDim.x) cnt[(size_t)k * nb + blockIdx.x] = c[k];
+    for (int k = threadIdx.x; k < kBuckets<SUB>; k += blockDim.x) cnt[(size_t)k * nb + blockIdx.x] = c[k];
 }
 
 // A block per tile of kPermTile rows, 256 rows at a time: each warp ranks its
@@ -42,20 +49,21 @@ __global__ void k_bucket_count(uint32_t n, const uint32_t *rp, uint32_t nb, uint
 // new ids.  Rows keep their order inside a class: stable, deterministic.
 constexpr int kPermThreads = 256;
 
+template <int SUB>
 __global__ void __launch_bounds__(kPermThreads) k_bucket_scatter(uint32_t n, const uint32_t *rp, uint32_t nb,
                                                                  const uint32_t *off, uint32_t *perm, uint32_t *inv) {
     constexpr int kWarps = kPermThreads / 32;
-    __shared__ uint32_t pos[kBuckets];
-    __shared__ uint32_t wc[kWarps][kBuckets];
+    __shared__ uint32_t pos[kBuckets<SUB>];
+    __shared__ uint32_t wc[kWarps][kBuckets<SUB>];
     const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (threadIdx.x < kBuckets) pos[threadIdx.x] = off[(size_t)threadIdx.x * nb + blockIdx.x];
+    for (int k = threadIdx.x; k < kBuckets<SUB>; k += kPermThreads) pos[k] = off[(size_t)k * nb + blockIdx.x];
     const uint64_t t0 = (uint64_t)blockIdx.x * kPermTile;
-    for (uint32_t c0 = 0; c0 < (uint32_t)kPermTile; c0 += kPermThreads) {
-        for (int k = threadIdx.x; k < kWarps * kBuckets; k += kPermThreads) (&wc[0][0])[k] = 0;
+    for (uint32_t r0 = 0; r0 < (uint32_t)kPermTile; r0 += kPermThreads) {
+        for (int k = threadIdx.x; k < kWarps * kBuckets<SUB>; k += kPermThreads) (&wc[0][0])[k] = 0;
         __syncthreads();
-        const uint64_t i = t0 + c0 + threadIdx.x;
+        const uint64_t i = t0 + r0 + threadIdx.x;
         const bool valid = i < n;
-        const uint32_t k = valid ? deg_key(rp[i + 1] - rp[i]) : 0u;
+        const uint32_t k = valid ? deg_key<SUB>(rp[i + 1] - rp[i]) : 0u;
         const unsigned act = __ballot_sync(0xFFFFFFFFu, valid);
         uint32_t rank = 0;
         if (valid) {
@@ -64,14 +72,14 @@ __global__ void __launch_bounds__(kPermThreads) k_bucket_scatter(uint32_t n, con
             if ((int)lane == __ffs(peers) - 1) wc[wid][k] = __popc(peers);
         }
         __syncthreads();
-        if (threadIdx.x < kBuckets) {
-            uint32_t t = pos[threadIdx.x];
+        for (int c0 = threadIdx.x; c0 < kBuckets<SUB>; c0 += kPermThreads) {
+            uint32_t t = pos[c0];
             for (int w = 0; w < kWarps; w++) {
-                const uint32_t c = wc[w][threadIdx.x];
-                wc[w][threadIdx.x] = t;
+                const uint32_t c = wc[w][c0];
+                wc[w][c0] = t;
                 t += c;
             }
-            pos[threadIdx.x] = t;
+            pos[c0] = t;
         }
         __syncthreads();
         if (valid) {
@@ -151,20 +159,35 @@ __global__ void k_max_u32(uint64_t m, const uint32_t *w, uint32_t *out) {
     if ((threadIdx.x & 31) == 0 && mx) atomicMax(out, mx);
 }
 
+// perm (vertex -> new id) and inv of the order by descending degree class,
+// stable inside a class
+template <int SUB>
+static int order_by_degree(Context &C, uint32_t n, const uint32_t *rp, uint32_t **perm, uint32_t **inv) {
+    const uint32_t nb = cdiv(n, kPermTile);
+    uint32_t *cnt, *off;
+    SGPB_TRY(dalloc_t(C, &cnt, (size_t)nb * kBuckets<SUB> + 1));
+    SGPB_TRY(dalloc_t(C, &off, (size_t)nb * kBuckets<SUB> + 1));
+    SGPB_TRY(dalloc_t(C, perm, n));
+    SGPB_TRY(dalloc_t(C, inv, n));
+    k_bucket_count<SUB><<<nb, 256, 0, C.stream>>>(n, rp, nb, cnt);
+    SGPB_TRY(scan_u32(C, cnt, off, nb * kBuckets<SUB>, nullptr));
+    k_bucket_scatter<SUB><<<nb, kPermThreads, 0, C.stream>>>(n, rp, nb, off, *perm, *inv);
+    C.kernel_launches += 2;
+    SGPB_CUDA(cudaGetLastError());
+    return SGP_B200_OK;
+}
+
+int degree_order(Context &C, uint32_t n, const uint32_t *rp, uint32_t **perm, uint32_t **inv) {
+    return order_by_degree<3>(C, n, rp, perm, inv);
+}
+
 int hub_first_copy(Context &C, const Level &L, uint32_t **perm_out, uint32_t **inv_out, Level *out) {
     const uint32_t n = L.n;
-    const uint32_t nb = cdiv(n, kPermTile);
-    uint32_t *cnt, *off, *perm, *inv, *deg;
-    SGPB_TRY(dalloc_t(C, &cnt, (size_t)nb * kBuckets + 1));
-    SGPB_TRY(dalloc_t(C, &off, (size_t)nb * kBuckets + 1));
-    SGPB_TRY(dalloc_t(C, &perm, n));
-    SGPB_TRY(dalloc_t(C, &inv, n));
+    uint32_t *perm, *inv, *deg;
     SGPB_TRY(dalloc_t(C, &deg, (size_t)n + 1));
-    k_bucket_count<<<nb, 256, 0, C.stream>>>(n, L.rp, nb, cnt);
-    SGPB_TRY(scan_u32(C, cnt, off, nb * kBuckets, nullptr));
-    k_bucket_scatter<<<nb, kPermThreads, 0, C.stream>>>(n, L.rp, nb, off, perm, inv);
+    SGPB_TRY(order_by_degree<0>(C, n, L.rp, &perm, &inv));
     k_perm_degrees<<<cdiv(n, 256), 256, 0, C.stream>>>(n, L.rp, inv, deg);
-    C.kernel_launches += 3;
+    C.kernel_launches++;
     *out = L;
     out->vcmap = nullptr;
     SGPB_TRY(dalloc_t(C, &out->rp, (size_t)n + 1));

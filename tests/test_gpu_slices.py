@@ -1,0 +1,132 @@
+"""Power iteration on row slices (slices.cu) at the edges of its forms: the
+iterate in one block's shared memory (up to 25,600 vertices), column panels
+(wider levels of at least two entries per row and panel) and the global
+gather; rows of every lane split, rows of several chunks and of several layout
+items, unit, repeated, 8-, 16-, 32- and 64-bit weights, rows without entries.
+Against the oracle after a fixed number of iterations: each iteration rounds
+the FP64 iterate to about 1e-16 per operation, so 40 of them stay well within
+1e-11 of its norm."""
+import numpy as np
+import pytest
+
+from ipdps_2021_graph_coarsening_b200 import graphs as G
+from oracle import bindings as O
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+CAP = 40
+
+
+def dev(a, wide=False):
+    t = np.uint64 if wide else np.uint32
+    return torch.from_numpy(np.ascontiguousarray(a, t).view(np.int64 if wide else np.int32)).cuda()
+
+
+def check(partitioner, rp, col, w=None, wide=False, cap=CAP):
+    n = rp.shape[0] - 1
+    x0 = np.random.default_rng(n).random(n)
+    u_o, it_o, lam_o = O.power_iter(rp, col, w, x0, 0.0, cap)
+    u, it, lam, _ = partitioner.power_iter(dev(rp), dev(col), None if w is None else dev(w, wide),
+                                           torch.from_numpy(x0).cuda(), None, 0.0, cap)
+    assert it == it_o == cap
+    assert np.linalg.norm(u.cpu().numpy() - u_o) <= 1e-11
+    assert abs(lam - lam_o) <= 1e-10 * abs(lam_o)
+
+
+def csr(n, u, v, w=None):
+    """Symmetric CSR of the given pairs (sorted rows, duplicates merged)."""
+    keep = u != v
+    u, v = u[keep], v[keep]
+    key = np.unique(np.concatenate([u.astype(np.int64) * n + v, v.astype(np.int64) * n + u]))
+    rows, cols = key // n, key % n
+    rp = np.zeros(n + 1, np.uint32)
+    rp[1:] = np.cumsum(np.bincount(rows, minlength=n))
+    return rp, cols.astype(np.uint32)
+
+
+def weights(rp, col, top, seed=1):
+    """Symmetric weights in [1, top] with both ends present."""
+    n = rp.shape[0] - 1
+    rows = np.repeat(np.arange(n, dtype=np.uint64), np.diff(rp).astype(np.int64))
+    lo, hi = np.minimum(rows, col), np.maximum(rows, col)
+    h = (lo * np.uint64(0x9E3779B97F4A7C15) ^ hi * np.uint64(0xC2B2AE3D27D4EB4F)) >> np.uint64(11)
+    w = 1 + h % np.uint64(top)
+    e = int(np.flatnonzero((rows == lo) & (col == hi))[0])
+    w[(lo == lo[e]) & (hi == hi[e])] = top
+    return w
+
+
+def skewed(n, m, seed):
+    """Power-law ends, a hub joined to every fourth vertex, the last vertices
+    without entries."""
+    rng = np.random.default_rng(seed)
+    u = (n * 0.97 * rng.random(m) ** 4).astype(np.int64)
+    v = (n * 0.97 * rng.random(m) ** 2).astype(np.int64)
+    hub = np.arange(1, int(n * 0.97), 4)
+    return csr(n, np.concatenate([u, np.zeros(hub.size, np.int64)]), np.concatenate([v, hub]))
+
+
+@pytest.mark.parametrize("n,m", [(4001, 30000), (25600, 400000), (25601, 400000), (51203, 1500000), (77000, 200000)])
+@pytest.mark.parametrize("top", [0, 200, 60000, 1 << 31])
+def test_forms_and_weights(partitioner, n, m, top):
+    """One panel exactly full, one vertex more, three panels, and a sparse
+    level (global gather), unit weights and every weight width."""
+    rp, col = skewed(n, m, n)
+    check(partitioner, rp, col, weights(rp, col, top) if top else None)
+
+
+def test_wide_weights(partitioner):
+    for n, m in ((9000, 120000), (60000, 900000)):
+        rp, col = skewed(n, m, 3)
+        check(partitioner, rp, col, weights(rp, col, (1 << 33) + 5), wide=True)
+
+
+def test_repeated_weights(partitioner):
+    """Panels of a level whose total weight is within 1.25 of its entries:
+    entries are repeated (several copies of one destination in a row)."""
+    rp, col = skewed(70001, 2000000, 5)
+    w = weights(rp, col, 9)
+    w[w < 9] = 1
+    w[w == 9] = np.where(np.isin(col[w == 9] % 2, (0,)), 1, 1)
+    rows = np.repeat(np.arange(70001), np.diff(rp).astype(np.int64))
+    w[(rows % 64 == 0) & (col % 64 == 0)] = 37
+    assert w.sum() <= 1.25 * w.size and w.max() == 37
+    check(partitioner, rp, col, w)
+
+
+@pytest.mark.parametrize("n", [9001, 60001])
+def test_long_rows(partitioner, n):
+    """Two hubs joined to every vertex: rows of several chunks and of several
+    layout items, beside rows of a few entries."""
+    i = np.arange(2, n)
+    rng = np.random.default_rng(n)
+    u = np.concatenate([np.zeros(n - 2, np.int64), np.ones(n - 2, np.int64), rng.integers(0, n, 4 * n)])
+    v = np.concatenate([i, i, rng.integers(0, n, 4 * n)])
+    rp, col = csr(n, u, v)
+    assert np.diff(rp).max() >= n - 2
+    check(partitioner, rp, col)
+    check(partitioner, rp, col, weights(rp, col, 1000))
+
+
+@pytest.mark.parametrize("name", ["grid", "er", "rgg"])
+def test_meshes(partitioner, name):
+    g = {"grid": lambda: G.grid2d(300, 211), "er": lambda: G.erdos_renyi(90001, 8.0, seed=3),
+         "rgg": lambda: G.rgg3d(30011, seed=2)}[name]()
+    check(partitioner, g.row_ptr, g.col)
+
+
+def test_finest_level_continues_on_slices(partitioner, monkeypatch):
+    """A finest level of at least 2^20 entries that does not stop after its
+    first iterations goes on from their iterate: the iteration count, the
+    value and the partition agree with the run on the main kernel alone."""
+    g = G.erdos_renyi(150001, 8.0, seed=9)
+    assert g.m_directed >= 1 << 20
+    a = partitioner.partition(g, rng_state=5)
+    monkeypatch.setenv("SGPB_PI_SLICES", "0")
+    b = partitioner.partition(g, rng_state=5)
+    assert a.level_n == b.level_n and a.level_iters[0] > 4
+    assert all(abs(x - y) <= 2 for x, y in zip(a.level_iters, b.level_iters))
+    assert abs(a.lam - b.lam) <= 1e-9 * abs(b.lam)
+    assert abs(a.edgecut - b.edgecut) <= 0.001 * b.edgecut
