@@ -1468,6 +1468,243 @@ __device__ __forceinline__ void small_level(const PIArgs &a) {
     }
 }
 
+// The FP64 small levels of runs without mixed precision.  An iteration of
+// small_level is a chain of block-wide barriers and five-value reductions on
+// 32 warps, about 2 us whatever the level's size.  Here a row has G lanes, G
+// chosen so that the rows fill the block once where they can; only the warps
+// with rows take part, behind a barrier of their own (one warp: none); each
+// thread's first kHeld entries stay in registers; and the three sums that the
+// recurrence needs are reduced once per warp, exchanged through shared memory
+// and combined by every warp for itself, so an iteration has one barrier.  The
+// fifth sum (u.u, for the eigenvalue) is taken once, at the end.  What is left
+// is the chain of a gather (65 clocks), the sums' shuffles (218 for the three)
+// and the reciprocal root (78).  24 vertices: 2.29 -> 0.63 us an iteration, 239
+// vertices 2.43 -> 1.25, 773 vertices 3.34 -> 1.94, 528 vertices of 13 entries a
+// row 11.8 -> 3.4.
+constexpr int kHeld = 8;
+
+template <typename W>
+__device__ __noinline__ void small_level_rows(const PIArgs &a) {
+    __shared__ double sm[256];
+    __shared__ double s_part[2][32][3];
+    extern __shared__ __align__(16) unsigned char dyn_smem[];
+    const uint32_t n = a.n;
+    const uint32_t m = (uint32_t)a.m;
+    const W *wg = (const W *)a.w;
+    // the arrays of small_level_bytes, at offsets from the block's shared
+    // memory (a pointer rounded as an integer would be a generic one)
+    const uint32_t o_col = (n + 1) * 4;
+    uint32_t o_w = (o_col + m * 4 + 15) & ~15u;
+    const uint32_t o_deg = wg ? (o_w + m * (uint32_t)sizeof(W) + 15) & ~15u : o_w;
+    const uint32_t o_xa = o_deg + n * 8, o_xb = o_xa + ((n * 8 + 15) & ~15u);
+    uint32_t *rp = (uint32_t *)dyn_smem;
+    uint32_t *col = (uint32_t *)(dyn_smem + o_col);
+    W *w = (W *)(dyn_smem + o_w);
+    double *deg = (double *)(dyn_smem + o_deg);
+    double *xa = (double *)(dyn_smem + o_xa);
+    double *xb = (double *)(dyn_smem + o_xb);
+    const uint32_t tid = threadIdx.x;
+    const unsigned lane = tid & 31, wid = tid >> 5;
+    for (uint32_t i = tid; i <= n; i += kSmallThreads) rp[i] = a.rp[i];
+    for (uint32_t j = tid; j < m; j += kSmallThreads) {
+        col[j] = a.col[j];
+        if (wg) w[j] = wg[j];
+    }
+    __syncthreads();
+    // start vector, weighted degrees, longest row
+    double p_sum = 0, p_maxd = 0;
+    uint32_t len_max = 0;
+    for (uint32_t i = tid; i < n; i += kSmallThreads) {
+        const uint32_t b = rp[i], e = rp[i + 1];
+        double d = (double)(e - b);
+        if (wg) {
+            uint64_t s = 0;
+            for (uint32_t j = b; j < e; j++) s += (uint64_t)w[j];
+            d = (double)s;
+        }
+        deg[i] = d;
+        p_maxd = d > p_maxd ? d : p_maxd;
+        len_max = e - b > len_max ? e - b : len_max;
+        const double x = a.vcmap ? a.x_in[a.vcmap[i]] : a.x_in[i];
+        xa[i] = x;
+        p_sum += x;
+    }
+    double v1[1] = {p_sum};
+    block_sum_d<1>(v1, sm);
+    p_maxd = warp_max(p_maxd);
+    const uint32_t wl = __reduce_max_sync(0xFFFFFFFFu, len_max);
+    if (lane == 0) {
+        sm[64 + wid] = p_maxd;
+        sm[96 + wid] = (double)wl;
+    }
+    if (tid == 0) sm[128] = v1[0];
+    __syncthreads();
+    const double S1 = sm[128];
+    const double maxd = warp_max(sm[64 + lane]);
+    len_max = (uint32_t)warp_max(sm[96 + lane]);
+    __syncthreads();
+    double gb = 2.0 * maxd;
+    if (gb < 2.0) gb = 2.0;
+    double mu = S1 / (double)n;
+    double q[1] = {0};
+    for (uint32_t i = tid; i < n; i += kSmallThreads) {
+        const double x = xa[i] - mu;
+        q[0] += x * x;
+    }
+    block_sum_d<1>(q, sm);
+    if (tid == 0) sm[128] = q[0];
+    __syncthreads();
+    double inv_nu = 1.0 / sqrt(sm[128]);
+    // lanes per row: the least of (rows after the first of a thread) * mean +
+    // longest row, per lane, and fixed prices of a row, a butterfly step (three
+    // entries' time) and the barrier of several warps
+    uint32_t lg = 0;
+    {
+        uint32_t best = 0xFFFFFFFFu;
+        const uint32_t avg = m / n + 1;
+        for (uint32_t g = 0; g <= 5; g++) {
+            const uint32_t passes = ((n << g) + kSmallThreads - 1) / kSmallThreads;
+            const uint32_t cost = (((passes - 1) * avg + len_max) >> g) + passes * (4 + 3 * g) +
+                                  ((n << g) > 32 ? 6 : 0);
+            if (cost < best) {
+                best = cost;
+                lg = g;
+            }
+        }
+    }
+    const uint32_t G = 1u << lg;
+    const uint32_t act = (n << lg) < kSmallThreads ? (((n << lg) + 31) & ~31u) : kSmallThreads;   // active threads
+    if (tid < act) {
+        const uint32_t nw = act / 32, g = tid & (G - 1), row0 = tid >> lg, step = act >> lg;
+        const uint32_t passes = (n + step - 1) / step;
+        // the first row's first entries of this lane
+        uint32_t hc[kHeld];
+        double hw[kHeld];
+        const uint32_t b0 = row0 < n ? rp[row0] : 0u, e0 = row0 < n ? rp[row0 + 1] : 0u;
+#pragma unroll
+        for (int k = 0; k < kHeld; k++) {
+            const uint32_t j = b0 + g + (k << lg);
+            const bool in = j < e0;
+            hc[k] = in ? col[j] : 0u;
+            hw[k] = in ? (wg ? (double)w[j] : 1.0) : 0.0;
+        }
+        const bool one = g == 0 && row0 < n;   // this lane ends row0
+        const double d0 = one ? deg[row0] : 0.0;
+        const uint32_t r0 = one ? row0 : 0u, j0 = b0 + g + (kHeld << lg);
+        const double rn = 1.0 / (double)n;
+        double dot = 0, last = 0;
+        uint64_t niter = 0;
+        double *src = xa, *dst = xb;
+        int buf = 0;
+        double s_ur = 0;
+        while (true) {
+            double P0 = 0, P1 = 0, P2 = 0;
+            auto fin = [&](uint32_t i, double acc, double ui, double d) {
+                const double r = next_value<false>(0, gb, mu, inv_nu, ui, acc, d);
+                dst[i] = r;
+                P0 += r;
+                P1 += r * r;
+                P2 += ui * r;
+            };
+            // entries j, j + G, ... < e from shared memory, two in flight
+            auto rest = [&](uint32_t j, uint32_t e, double &s, double &s1) {
+                if (wg) {
+                    for (; j + G < e; j += 2 * G) {
+                        s = fma((double)w[j], src[col[j]], s);
+                        s1 = fma((double)w[j + G], src[col[j + G]], s1);
+                    }
+                    if (j < e) s = fma((double)w[j], src[col[j]], s);
+                } else {
+                    for (; j + G < e; j += 2 * G) {
+                        s += src[col[j]];
+                        s1 += src[col[j + G]];
+                    }
+                    if (j < e) s += src[col[j]];
+                }
+            };
+            {
+                const double ui = (src[r0] - mu) * inv_nu;
+                double s = 0, s1 = 0;
+#pragma unroll
+                for (int k = 0; k < kHeld; k += 2) {
+                    s = fma(hw[k], src[hc[k]], s);
+                    s1 = fma(hw[k + 1], src[hc[k + 1]], s1);
+                }
+                rest(j0, e0, s, s1);
+                s += s1;
+                for (uint32_t o = 1; o < G; o <<= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+                if (one) fin(row0, s, ui, d0);
+            }
+            for (uint32_t ps = 1, i = row0 + step; ps < passes; ps++, i += step) {
+                double s = 0, s1 = 0;
+                rest(i < n ? rp[i] + g : 0u, i < n ? rp[i + 1] : 0u, s, s1);
+                s += s1;
+                for (uint32_t o = 1; o < G; o <<= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+                if (g == 0 && i < n) fin(i, s, (src[i] - mu) * inv_nu, deg[i]);
+            }
+            double t = warp_sum3(P0, P1, P2);
+            double A, B;
+            if (nw == 1) {
+                __syncwarp();
+                A = __shfl_sync(0xFFFFFFFFu, t, 0);
+                B = __shfl_sync(0xFFFFFFFFu, t, 1);
+                s_ur = __shfl_sync(0xFFFFFFFFu, t, 2);
+            } else {
+                if (lane < 3) s_part[buf][wid][lane] = t;
+                asm volatile("bar.sync 1, %0;" ::"r"(act) : "memory");
+                if (nw <= 4) {
+                    // few enough to add up from broadcast reads
+                    A = B = s_ur = 0;
+                    for (uint32_t k = 0; k < nw; k++) {
+                        A += s_part[buf][k][0];
+                        B += s_part[buf][k][1];
+                        s_ur += s_part[buf][k][2];
+                    }
+                } else {
+                    const bool in = lane < nw;
+                    t = warp_sum3(in ? s_part[buf][lane][0] : 0.0, in ? s_part[buf][lane][1] : 0.0,
+                                  in ? s_part[buf][lane][2] : 0.0);
+                    A = __shfl_sync(0xFFFFFFFFu, t, 0);
+                    B = __shfl_sync(0xFFFFFFFFu, t, 1);
+                    s_ur = __shfl_sync(0xFFFFFFFFu, t, 2);
+                }
+                buf ^= 1;
+            }
+            const double mu_n = A * rn;
+            const double inv_n = rsqrt(B - mu_n * A);
+            last = dot;
+            dot = s_ur * inv_n;
+            niter++;
+            const double delta = fabs(dot - last);
+            if (!(delta > a.tol && niter < a.iter_max)) break;
+            mu = mu_n;
+            inv_nu = inv_n;
+            double *x = src; src = dst; dst = x;
+        }
+        // u of the last iteration and its norm
+        double uu = 0;
+        for (uint32_t i = tid; i < n; i += act) {
+            const double u = (src[i] - mu) * inv_nu;
+            a.out[i] = u;
+            uu += u * u;
+        }
+        double t = warp_sum3(uu, 0, 0);
+        if (nw > 1) {
+            if (lane == 0) s_part[buf][wid][0] = t;
+            asm volatile("bar.sync 1, %0;" ::"r"(act) : "memory");
+            t = warp_sum3(lane < nw ? s_part[buf][lane][0] : 0.0, 0, 0);
+        }
+        if (tid == 0) {
+            a.res[0] = (double)niter;
+            a.res[1] = dot;
+            a.res[2] = gb;
+            a.res[3] = (gb * t - s_ur) / t;
+            a.res[4] = niter >= a.iter_max ? 1.0 : 0.0;
+            a.res[5] = 0.0;
+        }
+    }
+}
+
 template <typename W, typename V>
 __global__ void __launch_bounds__(kSmallThreads, 1) k_power_iter_small(PIArgs a) {
     small_level<W, V>(a);
@@ -1478,6 +1715,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_power_iter_small(PIArgs a)
 struct PIChainDesc {
     PIArgs a;
     int wbytes;   // 0, 4 or 8
+    int rows;     // small_level_rows
 };
 
 // Work queue over chains (the host orders them largest first): each block
@@ -1499,8 +1737,14 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_power_iter_chains(const PI
         for (uint32_t k = 0; k < ch.y; k++) {
             const PIChainDesc &d = lev[ch.x + k];
             const unsigned long long t0 = global_ns();
-            if (d.wbytes == 8) small_level<unsigned long long, double>(d.a);
-            else small_level<uint32_t, double>(d.a);
+            if (d.rows) {
+                if (d.wbytes == 8) small_level_rows<unsigned long long>(d.a);
+                else small_level_rows<uint32_t>(d.a);
+            } else if (d.wbytes == 8) {
+                small_level<unsigned long long, double>(d.a);
+            } else {
+                small_level<uint32_t, double>(d.a);
+            }
             // the result is visible to the next level, and shared memory free
             __syncthreads();
             if (threadIdx.x == 0) d.a.res[6] = (double)(global_ns() - t0) * 1e-6;
@@ -2605,6 +2849,10 @@ int power_iter_chains(Context &C, const std::vector<PIChain *> &chains, const Po
             d.a.iter_max = iter_budget(L.n, o);
             d.a.normlap = o.normlap;
             d.wbytes = L.wbytes;
+            // mixed runs and the normalized walk keep small_level's order of
+            // sums: the FP32 differences of a mixed run's larger levels, and
+            // the walk without deflation, amplify any other rounding
+            d.rows = !o.mixed && !o.normlap;
             h.push_back(d);
             cost += L.m + 8ull * L.n;
             const size_t b = L.wbytes == 8 ? small_level_bytes<unsigned long long, double>(L.n, L.m, L.w != nullptr)

@@ -23,6 +23,26 @@ __device__ __forceinline__ double next_value(int normlap, double gb, double mu, 
     }
 }
 
+// Sum of three values over a warp, packed: value k of the warp ends up in
+// lanes with (lane & 3) == k (k < 3).  6 double shuffles instead of 15.
+__device__ __forceinline__ double warp_sum3(double a, double b, double c) {
+    const unsigned lane = threadIdx.x & 31;
+    const bool o1 = lane & 1, o2 = lane & 2;
+    // step 1: even lanes keep (a, c), odd lanes keep (b, 0)
+    double k0 = o1 ? b : a, s0 = o1 ? a : b;
+    double k1 = o1 ? 0.0 : c, s1 = o1 ? c : 0.0;
+    k0 += __shfl_xor_sync(0xFFFFFFFFu, s0, 1);
+    k1 += __shfl_xor_sync(0xFFFFFFFFu, s1, 1);
+    // step 2: lanes without bit 1 keep k0, the others k1
+    double v = o2 ? k1 : k0;
+    const double s = o2 ? k0 : k1;
+    v += __shfl_xor_sync(0xFFFFFFFFu, s, 2);
+    v += __shfl_xor_sync(0xFFFFFFFFu, v, 4);
+    v += __shfl_xor_sync(0xFFFFFFFFu, v, 8);
+    v += __shfl_xor_sync(0xFFFFFFFFu, v, 16);
+    return v;
+}
+
 // mbarriers and 1-D bulk copies into shared memory
 constexpr uint32_t kMbarWaitLimit = 1u << 22;   // polls before giving up
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }

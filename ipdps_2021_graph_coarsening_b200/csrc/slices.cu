@@ -128,26 +128,6 @@ struct GridBar {
     }
 };
 
-// Sum of three values over a warp, packed: value k of the warp ends up in
-// lanes with (lane & 3) == k (k < 3).  6 double shuffles instead of 15.
-__device__ __forceinline__ double warp_sum3(double a, double b, double c) {
-    const unsigned lane = threadIdx.x & 31;
-    const bool o1 = lane & 1, o2 = lane & 2;
-    // step 1: even lanes keep (a, c), odd lanes keep (b, 0)
-    double k0 = o1 ? b : a, s0 = o1 ? a : b;
-    double k1 = o1 ? 0.0 : c, s1 = o1 ? c : 0.0;
-    k0 += __shfl_xor_sync(0xFFFFFFFFu, s0, 1);
-    k1 += __shfl_xor_sync(0xFFFFFFFFu, s1, 1);
-    // step 2: lanes without bit 1 keep k0, the others k1
-    double v = o2 ? k1 : k0;
-    const double s = o2 ? k0 : k1;
-    v += __shfl_xor_sync(0xFFFFFFFFu, s, 2);
-    v += __shfl_xor_sync(0xFFFFFFFFu, v, 4);
-    v += __shfl_xor_sync(0xFFFFFFFFu, v, 8);
-    v += __shfl_xor_sync(0xFFFFFFFFu, v, 16);
-    return v;
-}
-
 // The block's sums of p[3], written to dst[0..2] by warp 0 (sm: 3 x 32).
 __device__ __forceinline__ void block_sum3_to(const double (&p)[kSumK], double (*sm)[kSumK], double *dst) {
     const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;

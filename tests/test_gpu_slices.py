@@ -27,9 +27,10 @@ def dev(a, wide=False):
 def check(partitioner, rp, col, w=None, wide=False, cap=CAP):
     n = rp.shape[0] - 1
     x0 = np.random.default_rng(n).random(n)
-    u_o, it_o, lam_o = O.power_iter(rp, col, w, x0, 0.0, cap)
+    # a negative tolerance: no iterate, converged or not, stops before the cap
+    u_o, it_o, lam_o = O.power_iter(rp, col, w, x0, -1.0, cap)
     u, it, lam, _ = partitioner.power_iter(dev(rp), dev(col), None if w is None else dev(w, wide),
-                                           torch.from_numpy(x0).cuda(), None, 0.0, cap)
+                                           torch.from_numpy(x0).cuda(), None, -1.0, cap)
     assert it == it_o == cap
     assert np.linalg.norm(u.cpu().numpy() - u_o) <= 1e-11
     assert abs(lam - lam_o) <= 1e-10 * abs(lam_o)
@@ -130,3 +131,27 @@ def test_finest_level_continues_on_slices(partitioner, monkeypatch):
     assert all(abs(x - y) <= 2 for x, y in zip(a.level_iters, b.level_iters))
     assert abs(a.lam - b.lam) <= 1e-9 * abs(b.lam)
     assert abs(a.edgecut - b.edgecut) <= 0.001 * b.edgecut
+
+
+@pytest.mark.parametrize("n", [5, 31, 32, 33, 64, 129, 600, 1023, 1025, 1900])
+@pytest.mark.parametrize("top", [0, 50])
+def test_small_levels(partitioner, n, top):
+    """Levels of one block: one warp, several warps, every lane split, more
+    rows than threads, with a hub row beside short ones, unit and integer
+    weights."""
+    rng = np.random.default_rng(n)
+    i = np.arange(n - 1)
+    hub = np.arange(1, n, 3)
+    u = np.concatenate([i, np.zeros(hub.size, np.int64), rng.integers(0, n, 2 * n)])
+    v = np.concatenate([i + 1, hub, rng.integers(0, n, 2 * n)])
+    rp, col = csr(n, u, v)
+    assert rp[-1] + 8 * n <= 32768
+    check(partitioner, rp, col, weights(rp, col, top) if top else None)
+
+
+def test_small_level_dense(partitioner):
+    """A small level of long rows: many lanes a row."""
+    rng = np.random.default_rng(7)
+    rp, col = csr(90, rng.integers(0, 90, 9000), rng.integers(0, 90, 9000))
+    check(partitioner, rp, col, weights(rp, col, 1000))
+    check(partitioner, rp, col, weights(rp, col, (1 << 33) + 1), wide=True)
