@@ -348,7 +348,7 @@ int sgp_b200_split(sgp_b200_ctx_t *ctx, uint32_t n, const uint32_t *row_ptr, con
  * of the call (a host application that owns every device allocation through
  * its own pool, code running in an out-of-memory handler, a plug-in whose
  * host forbids allocation): it allocates nothing and uses a fixed scratch
- * array inside the library (about 8 MiB per GPU, held until the process
+ * array inside the library (about 4 MiB per GPU, held until the process
  * exits).  At most SGP_B200_NOALLOC_MAX_N vertices; larger graphs return
  * SGP_B200_ERR_TOO_LARGE.  Asynchronous on `stream` (a cudaStream_t, NULL =
  * default stream): part (n entries) and result (device array: result[0] =

@@ -26,6 +26,9 @@
 // Passes repeat until one applies nothing or leaves the cut unchanged.
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
+#include "bits.cuh"
 #include "common.cuh"
 #include "internal.h"
 
@@ -34,52 +37,89 @@ namespace cg = cooperative_groups;
 namespace sgpb {
 
 constexpr int kFmBuckets = 1024;
-constexpr uint32_t kFmNone = 0xFFFFFFFFu;
 constexpr int kFmTile = 1024;   // candidates per block in the counting sort
 
-// gains, candidate flags, cut and balance.  Unit edge weights (the finest
+// Gains, candidate flags, cut and balance.  Unit edge weights (the finest
 // level): a symmetric graph with fewer than 2^32 directed entries has every
-// degree below 2^31, so 32-bit sums are exact.  G lanes per row, four
-// entries per lane in flight (destinations, then the part gathers).
-template <int G>
-__global__ void __launch_bounds__(256) k_fm_gain(uint32_t n, const uint32_t *__restrict__ rp,
-                                                 const uint32_t *__restrict__ col,
-                                                 const uint32_t *__restrict__ part, long long *__restrict__ gain,
-                                                 uint8_t *__restrict__ f0, uint8_t *__restrict__ f1,
-                                                 unsigned long long *__restrict__ sums /* [0] 2 cut, [1] bal */) {
-    const unsigned gm = group_mask<G>();
-    const uint32_t lane = threadIdx.x & (G - 1);
-    const uint64_t ng = ((uint64_t)gridDim.x * blockDim.x) / G;
+// degree below 2^31, so 32-bit sums are exact.  The parts are a bitmap, in
+// the block's shared memory when it fits (SHARED); rows of more than kLongRow
+// entries take a block each, the others G lanes each with four entries per
+// lane in flight.  R-MAT 18 (7.6M entries, hubs of 30,000): with parts
+// gathered through L1 and hub rows on a warp each 177 us a pass, now 24.
+struct FmGraph {
+    uint32_t n;
+    const uint32_t *rp, *col;
+    const uint32_t *bits;     // part 1
+    const uint32_t *longs;    // rows of more than kLongRow entries
+    const uint32_t *nlong;
+};
+
+template <int G, bool SHARED>
+__global__ void __launch_bounds__(1024) k_fm_gain(FmGraph a, long long *__restrict__ gain,
+                                                  uint32_t *__restrict__ flag /* [2n]: side 0, side 1 */,
+                                                  unsigned long long *__restrict__ sums /* [0] 2 cut, [1] balance,
+                                                                                           [2], [3] candidates */) {
+    extern __shared__ uint32_t s_bits[];
+    __shared__ int s_sum;
+    if (SHARED) bits_load(a.bits, bit_words(a.n), s_bits);
+    const uint32_t *bits = SHARED ? (const uint32_t *)s_bits : a.bits;
+    if (threadIdx.x == 0) s_sum = 0;
+    __syncthreads();
     unsigned long long cut2 = 0;
     long long bal = 0;
-    for (uint64_t u = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / G; u < n; u += ng) {
-        const uint32_t pu = __ldg(part + u);
-        const uint32_t b = __ldg(rp + u), e = __ldg(rp + u + 1);
+    uint32_t c0 = 0, c1 = 0;
+    auto done = [&](uint32_t u, uint32_t pu, int across, int deg) {
+        const int g = 2 * across - deg;   // across minus inside
+        gain[u] = g;
+        flag[u] = pu == 0 && g > 0;
+        flag[(size_t)a.n + u] = pu != 0 && g > 0;
+        c0 += pu == 0 && g > 0;
+        c1 += pu != 0 && g > 0;
+        cut2 += (unsigned)across;
+        bal += pu == 0 ? 1 : -1;
+    };
+    const uint32_t nl = *a.nlong;
+    for (uint32_t r = blockIdx.x; r < nl; r += gridDim.x) {
+        const uint32_t u = __ldg(a.longs + r), b = __ldg(a.rp + u), e = __ldg(a.rp + u + 1);
+        const uint32_t pu = bit_of(bits, u);
+        int across = 0;
+#pragma unroll 4
+        for (uint64_t j = (uint64_t)b + threadIdx.x; j < e; j += 1024) across += bit_of(bits, __ldg(a.col + j)) != pu;
+        across = __reduce_add_sync(0xFFFFFFFFu, across);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&s_sum, across);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            done(u, pu, s_sum, (int)(e - b));
+            s_sum = 0;
+        }
+        __syncthreads();
+    }
+    const uint32_t lane = threadIdx.x & (G - 1);
+    const uint64_t ng = ((uint64_t)gridDim.x * blockDim.x) / G;
+    for (uint64_t u = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / G; u < a.n; u += ng) {
+        const uint32_t b = __ldg(a.rp + u), e = __ldg(a.rp + u + 1);
+        if (e - b > kLongRow) continue;   // uniform in the row's group
+        const uint32_t pu = bit_of(bits, (uint32_t)u);
         int across = 0;
         for (uint32_t j0 = b + lane; j0 < e; j0 += 4 * G) {
             uint32_t v[4];
 #pragma unroll
-            for (int q = 0; q < 4; q++) v[q] = j0 + q * G < e ? __ldg(col + j0 + q * G) : 0xFFFFFFFFu;
+            for (int q = 0; q < 4; q++) v[q] = j0 + q * G < e ? __ldg(a.col + j0 + q * G) : (uint32_t)u;
 #pragma unroll
-            for (int q = 0; q < 4; q++)
-                if (v[q] != 0xFFFFFFFFu) across += __ldg(part + v[q]) != pu;
+            for (int q = 0; q < 4; q++) across += bit_of(bits, v[q]) != pu;
         }
         across = group_sum<G>(across);
-        if (lane == 0) {
-            const int deg = (int)(e - b);
-            const int g = 2 * across - deg;   // across minus inside
-            gain[u] = g;
-            f0[u] = pu == 0 && g > 0;
-            f1[u] = pu != 0 && g > 0;
-            cut2 += (unsigned)across;
-            bal += pu == 0 ? 1 : -1;
-        }
+        if (lane == 0) done((uint32_t)u, pu, across, (int)(e - b));
     }
     cut2 = warp_sum(cut2);
     bal = warp_sum(bal);
+    c0 = __reduce_add_sync(0xFFFFFFFFu, c0);
+    c1 = __reduce_add_sync(0xFFFFFFFFu, c1);
     if ((threadIdx.x & 31) == 0) {
         if (cut2) atomicAdd(sums, cut2);
         if (bal) atomicAdd(sums + 1, (unsigned long long)bal);
+        if (c0) atomicAdd(sums + 2, (unsigned long long)c0);
+        if (c1) atomicAdd(sums + 3, (unsigned long long)c1);
     }
 }
 
@@ -87,44 +127,56 @@ __device__ __forceinline__ uint32_t fm_bucket(long long g) {
     return g < kFmBuckets - 1 ? (uint32_t)g : (uint32_t)(kFmBuckets - 1);
 }
 
-// counts per (descending bucket, tile): hist[(kFmBuckets - 1 - b) * ntiles + t]
-__global__ void __launch_bounds__(kFmTile) k_fm_hist(uint32_t len, const uint32_t *__restrict__ idx,
+// flagged vertices in order (n2 = 2n flags: side 0 before side 1)
+__global__ void k_fm_list(uint32_t n2, const uint32_t *__restrict__ flag, const uint32_t *__restrict__ pos, uint32_t n,
+                          uint32_t *__restrict__ idx) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n2 && flag[i]) idx[pos[i]] = (uint32_t)(i < n ? i : i - n);
+}
+
+// Counting sort of both sides' candidates (the first na of the list are side
+// 0's): key = side, then the descending bucket.
+constexpr int kFmKeys = 2 * kFmBuckets;
+__device__ __forceinline__ uint32_t fm_key(uint32_t i, uint32_t na, long long g) {
+    return (i < na ? 0u : (uint32_t)kFmBuckets) + (uint32_t)(kFmBuckets - 1) - fm_bucket(g);
+}
+
+// counts per (key, tile): hist[key * ntiles + t]
+__global__ void __launch_bounds__(kFmTile) k_fm_hist(uint32_t len, uint32_t na, const uint32_t *__restrict__ idx,
                                                      const long long *__restrict__ gain, uint32_t ntiles,
                                                      uint32_t *__restrict__ hist) {
-    __shared__ uint32_t cnt[kFmBuckets];
-    for (int b = threadIdx.x; b < kFmBuckets; b += blockDim.x) cnt[b] = 0;
+    __shared__ uint32_t cnt[kFmKeys];
+    for (int b = threadIdx.x; b < kFmKeys; b += blockDim.x) cnt[b] = 0;
     __syncthreads();
     const uint32_t i = blockIdx.x * kFmTile + threadIdx.x;
-    if (i < len) atomicAdd(&cnt[fm_bucket(gain[idx[i]])], 1u);
+    if (i < len) atomicAdd(&cnt[fm_key(i, na, gain[idx[i]])], 1u);
     __syncthreads();
-    for (int b = threadIdx.x; b < kFmBuckets; b += blockDim.x)
-        hist[(size_t)(kFmBuckets - 1 - b) * ntiles + blockIdx.x] = cnt[b];
+    for (int b = threadIdx.x; b < kFmKeys; b += blockDim.x) hist[(size_t)b * ntiles + blockIdx.x] = cnt[b];
 }
 
 // stable placement: within a tile the warps take turns in order, and lanes
-// of one bucket rank by lane
-__global__ void __launch_bounds__(kFmTile) k_fm_place(uint32_t len, const uint32_t *__restrict__ idx,
+// of one key rank by lane
+__global__ void __launch_bounds__(kFmTile) k_fm_place(uint32_t len, uint32_t na, const uint32_t *__restrict__ idx,
                                                       const long long *__restrict__ gain, uint32_t ntiles,
                                                       const uint32_t *__restrict__ off,
                                                       uint32_t *__restrict__ sorted) {
-    __shared__ uint32_t cnt[kFmBuckets];
-    for (int b = threadIdx.x; b < kFmBuckets; b += blockDim.x) cnt[b] = 0;
+    __shared__ uint32_t cnt[kFmKeys];
+    for (int b = threadIdx.x; b < kFmKeys; b += blockDim.x) cnt[b] = 0;
     __syncthreads();
     const uint32_t i = blockIdx.x * kFmTile + threadIdx.x;
     const bool valid = i < len;
     const uint32_t u = valid ? idx[i] : 0u;
-    const uint32_t b = valid ? fm_bucket(gain[u]) : 0u;
+    const uint32_t b = valid ? fm_key(i, na, gain[u]) : 0u;
+    const uint32_t base = valid ? off[(size_t)b * ntiles + blockIdx.x] : 0u;
     const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const unsigned act = __ballot_sync(0xFFFFFFFFu, valid);
+    const unsigned peers = valid ? __match_any_sync(act, b) : 0u;
     for (unsigned turn = 0; turn < kFmTile / 32; turn++) {
-        if (wid == turn) {
-            const unsigned act = __ballot_sync(0xFFFFFFFFu, valid);
-            if (valid) {
-                const unsigned peers = __match_any_sync(act, b);
-                const uint32_t r = cnt[b] + __popc(peers & ((1u << lane) - 1u));
-                sorted[off[(size_t)(kFmBuckets - 1 - b) * ntiles + blockIdx.x] + r] = u;
-                __syncwarp(peers);
-                if ((int)lane == __ffs(peers) - 1) cnt[b] += __popc(peers);
-            }
+        if (wid == turn && valid) {
+            const uint32_t r = cnt[b] + __popc(peers & ((1u << lane) - 1u));
+            sorted[base + r] = u;
+            __syncwarp(peers);
+            if ((int)lane == __ffs(peers) - 1) cnt[b] += __popc(peers);
         }
         __syncthreads();
     }
@@ -134,7 +186,9 @@ __global__ void __launch_bounds__(kFmTile) k_fm_place(uint32_t len, const uint32
 __global__ void k_fm_interleave(uint32_t na, uint32_t nb, const uint32_t *__restrict__ A,
                                 const uint32_t *__restrict__ B, const long long *__restrict__ gain, long long d,
                                 uint32_t *__restrict__ order, uint32_t *__restrict__ rank,
-                                uint8_t *__restrict__ side) {
+                                uint32_t *__restrict__ listed, uint8_t *__restrict__ side,
+                                unsigned long long key0, unsigned long long *__restrict__ best) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *best = key0;   // k = 0
     // phase 1: ceil(|d| / 2) moves from the heavier side (as many as it has)
     const bool heavy0 = d > 0;
     const uint64_t want = d > 0 ? (uint64_t)(d + 1) / 2 : (uint64_t)(-d + 1) / 2;
@@ -170,34 +224,68 @@ __global__ void k_fm_interleave(uint32_t na, uint32_t nb, const uint32_t *__rest
             }
             order[pos] = u;
             rank[u] = (uint32_t)pos;
+            atomicOr(listed + (u >> 5), 1u << (u & 31u));
             side[pos] = (uint8_t)s;
         }
     }
 }
 
-// sequential gain of the i-th move (unit weights, 32-bit sums as above)
-template <int G>
-__global__ void __launch_bounds__(256) k_fm_seqgain(uint32_t k, const uint32_t *__restrict__ rp,
-                                                    const uint32_t *__restrict__ col,
-                                                    const uint32_t *__restrict__ part,
-                                                    const uint32_t *__restrict__ order,
-                                                    const uint32_t *__restrict__ rank, long long *__restrict__ gseq) {
+// Sequential gain of the i-th move (unit weights, 32-bit sums as above).  A
+// second bitmap says which vertices are listed, so ranks are read of those
+// alone.
+template <int G, bool SHARED>
+__global__ void __launch_bounds__(1024) k_fm_seqgain(FmGraph a, uint32_t k, const uint32_t *__restrict__ listed,
+                                                     const uint32_t *__restrict__ order,
+                                                     const uint32_t *__restrict__ rank, long long *__restrict__ gseq) {
+    extern __shared__ uint32_t s_bits[];
+    __shared__ int s_sum;
+    const uint32_t words = bit_words(a.n);
+    if (SHARED) {
+        bits_load(a.bits, words, s_bits);
+        bits_load(listed, words, s_bits + words);
+    }
+    const uint32_t *bits = SHARED ? (const uint32_t *)s_bits : a.bits;
+    const uint32_t *lst = SHARED ? (const uint32_t *)(s_bits + words) : listed;
+    if (threadIdx.x == 0) s_sum = 0;
+    __syncthreads();
+    // an entry counts +1: across xor moved before
+    auto term = [&](uint32_t v, uint32_t pu, uint32_t i) -> int {
+        const bool across = bit_of(bits, v) != pu;
+        const bool moved = bit_of(lst, v) && __ldg(rank + v) < i;
+        return across != moved;
+    };
+    const uint32_t nl = *a.nlong;
+    for (uint32_t r = blockIdx.x; r < nl; r += gridDim.x) {
+        const uint32_t u = __ldg(a.longs + r);
+        if (!bit_of(lst, u)) continue;   // uniform in the block
+        const uint32_t i = __ldg(rank + u), b = __ldg(a.rp + u), e = __ldg(a.rp + u + 1), pu = bit_of(bits, u);
+        int plus = 0;
+#pragma unroll 4
+        for (uint64_t j = (uint64_t)b + threadIdx.x; j < e; j += 1024) plus += term(__ldg(a.col + j), pu, i);
+        plus = __reduce_add_sync(0xFFFFFFFFu, plus);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&s_sum, plus);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            gseq[i] = 2 * s_sum - (int)(e - b);
+            s_sum = 0;
+        }
+        __syncthreads();
+    }
     const uint32_t lane = threadIdx.x & (G - 1);
     const uint64_t ng = ((uint64_t)gridDim.x * blockDim.x) / G;
     for (uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / G; i < k; i += ng) {
-        const uint32_t u = __ldg(order + i), pu = __ldg(part + u);
-        const uint32_t b = __ldg(rp + u), e = __ldg(rp + u + 1);
-        int plus = 0;   // neighbours counting +1: across xor moved before
+        const uint32_t u = __ldg(order + i);
+        const uint32_t b = __ldg(a.rp + u), e = __ldg(a.rp + u + 1);
+        if (e - b > kLongRow) continue;   // uniform in the row's group
+        const uint32_t pu = bit_of(bits, u);
+        int plus = 0;
         for (uint32_t j0 = b + lane; j0 < e; j0 += 4 * G) {
             uint32_t v[4];
 #pragma unroll
-            for (int q = 0; q < 4; q++) v[q] = j0 + q * G < e ? __ldg(col + j0 + q * G) : 0xFFFFFFFFu;
+            for (int q = 0; q < 4; q++) v[q] = j0 + q * G < e ? __ldg(a.col + j0 + q * G) : 0xFFFFFFFFu;
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                if (v[q] == 0xFFFFFFFFu) continue;
-                const bool across = __ldg(part + v[q]) != pu, moved = __ldg(rank + v[q]) < (uint32_t)i;
-                plus += across != moved;
-            }
+            for (int q = 0; q < 4; q++)
+                if (v[q] != 0xFFFFFFFFu) plus += term(v[q], pu, (uint32_t)i);
         }
         plus = group_sum<G>(plus);
         if (lane == 0) gseq[i] = 2 * plus - (int)(e - b);
@@ -269,9 +357,14 @@ __global__ void __launch_bounds__(256) k_fm_best(FmBestArgs a) {
     if ((threadIdx.x & 31) == 0 && best != ~0ull) atomicMin(a.best, best);
 }
 
-__global__ void k_fm_apply(uint32_t k, const uint32_t *__restrict__ order, uint32_t *__restrict__ part) {
+__global__ void k_fm_apply(uint32_t k, const uint32_t *__restrict__ order, uint32_t *__restrict__ part,
+                           uint32_t *__restrict__ bits) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < k; i += stride) part[order[i]] ^= 1u;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < k; i += stride) {
+        const uint32_t u = order[i];
+        part[u] ^= 1u;
+        atomicXor(bits + (u >> 5), 1u << (u & 31u));
+    }
 }
 
 static uint32_t fm_grid(Context &C, uint64_t items) {
@@ -286,26 +379,21 @@ static int fm_impl(Context &C, const Level &L, const W *w, uint32_t *part, uint3
                    uint32_t *passes_out, uint64_t *moves_out) {
     const uint32_t n = L.n;
     long long *gain, *gseq, *chunk_g, *chunk_b;
-    uint8_t *f0, *f1, *side;
-    uint32_t *A, *B, *sa, *sb, *order, *rank, *cnt, *hist, *off;
+    uint8_t *side;
+    uint32_t *flag, *pos, *idx, *sorted, *order, *rank, *hist = nullptr, *off = nullptr;
     unsigned long long *sums, *best;
     SGPB_TRY(dalloc_t(C, &gain, n));
     SGPB_TRY(dalloc_t(C, &gseq, n));
-    SGPB_TRY(dalloc_t(C, &f0, n));
-    SGPB_TRY(dalloc_t(C, &f1, n));
+    SGPB_TRY(dalloc_t(C, &flag, 2 * (size_t)n + 1));
+    SGPB_TRY(dalloc_t(C, &pos, 2 * (size_t)n + 1));
     SGPB_TRY(dalloc_t(C, &side, n));
-    SGPB_TRY(dalloc_t(C, &A, n));
-    SGPB_TRY(dalloc_t(C, &B, n));
-    SGPB_TRY(dalloc_t(C, &sa, n));
-    SGPB_TRY(dalloc_t(C, &sb, n));
+    SGPB_TRY(dalloc_t(C, &idx, n));
+    SGPB_TRY(dalloc_t(C, &sorted, n));
     SGPB_TRY(dalloc_t(C, &order, n));
     SGPB_TRY(dalloc_t(C, &rank, n));
-    SGPB_TRY(dalloc_t(C, &cnt, 2));
-    SGPB_TRY(dalloc_t(C, &sums, 2));
+    SGPB_TRY(dalloc_t(C, &sums, 4));
     SGPB_TRY(dalloc_t(C, &best, 1));
-    const uint32_t max_tiles = cdiv(n, kFmTile);
-    SGPB_TRY(dalloc_t(C, &hist, (size_t)kFmBuckets * max_tiles + 1));
-    SGPB_TRY(dalloc_t(C, &off, (size_t)kFmBuckets * max_tiles + 1));
+    uint32_t hist_tiles = 0;   // tiles hist and off have room for
     int per_sm = 0;
     SGPB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fm_best, 256, 0));
     if (per_sm < 1) {
@@ -316,46 +404,94 @@ static int fm_impl(Context &C, const Level &L, const W *w, uint32_t *part, uint3
     SGPB_TRY(dalloc_t(C, &chunk_g, bgrid_max));
     SGPB_TRY(dalloc_t(C, &chunk_b, bgrid_max));
     const double avg = n ? (double)L.m / n : 0;
+    // parts and listed vertices as bitmaps, the long rows' list
+    const uint32_t words = bit_words(n);
+    uint32_t *bits, *listed, *longs, *nlong;
+    SGPB_TRY(dalloc_t(C, &bits, words));
+    SGPB_TRY(dalloc_t(C, &listed, words));
+    SGPB_TRY(dalloc_t(C, &longs, n));
+    SGPB_TRY(dalloc_t(C, &nlong, 1));
+    SGPB_TRY(dzero(C, nlong, 4));
+    SGPB_TRY(part_bits(C, n, part, bits));
+    SGPB_TRY(long_rows(C, n, L.rp, longs, nlong));
+    const FmGraph fg{n, L.rp, L.col, bits, longs, nlong};
+    // blocks of 1024 threads: two an SM while their bitmaps fit
+    auto row_grid = [&](uint64_t threads, uint32_t smem_words) -> uint32_t {
+        const uint32_t cap = (uint32_t)C.num_sms * (smem_words <= kBitsMaxWords / 2 ? 2u : 1u);
+        const uint64_t g = (threads + 1023) / 1024;
+        return g > cap ? cap : g ? (uint32_t)g : 1u;
+    };
+    const bool sh1 = words <= kBitsMaxWords, sh2 = 2 * words <= kBitsMaxWords;
+    auto gain_pass = [&](auto gt) -> int {
+        constexpr int G = decltype(gt)::value;
+        const uint32_t g = row_grid((uint64_t)n * G, sh1 ? words : 0);
+        if (sh1) {
+            SGPB_CUDA(cudaFuncSetAttribute(k_fm_gain<G, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)(kBitsMaxWords * 4)));
+            k_fm_gain<G, true><<<g, 1024, (size_t)words * 4, C.stream>>>(fg, gain, flag, sums);
+        } else {
+            k_fm_gain<G, false><<<g, 1024, 0, C.stream>>>(fg, gain, flag, sums);
+        }
+        return SGP_B200_OK;
+    };
+    auto seq_pass = [&](auto gt, uint32_t k) -> int {
+        constexpr int G = decltype(gt)::value;
+        const uint32_t g = row_grid((uint64_t)k * G, sh2 ? 2 * words : 0);
+        if (sh2) {
+            SGPB_CUDA(cudaFuncSetAttribute(k_fm_seqgain<G, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)(kBitsMaxWords * 4)));
+            k_fm_seqgain<G, true><<<g, 1024, (size_t)words * 8, C.stream>>>(fg, k, listed, order, rank, gseq);
+        } else {
+            k_fm_seqgain<G, false><<<g, 1024, 0, C.stream>>>(fg, k, listed, order, rank, gseq);
+        }
+        return SGP_B200_OK;
+    };
+    // lanes for about a trip of four entries each a row
+    typedef std::integral_constant<int, 2> G2;
+    typedef std::integral_constant<int, 8> G8;
+    typedef std::integral_constant<int, 32> G32;
     uint64_t moves = 0;
     uint32_t pass = 0;
     for (; pass < max_passes; pass++) {
-        SGPB_TRY(dzero(C, sums, 2 * sizeof(unsigned long long)));
-#define SGPB_FMG(G) k_fm_gain<G><<<fm_grid(C, (uint64_t)n * G), 256, 0, C.stream>>>(n, L.rp, L.col, part, gain, f0, f1, sums)
-        if (avg <= 4) SGPB_FMG(4);
-        else if (avg <= 16) SGPB_FMG(16);
-        else SGPB_FMG(32);
-#undef SGPB_FMG
-        SGPB_TRY(compact_flags(C, f0, n, A, cnt));
-        SGPB_TRY(compact_flags(C, f1, n, B, cnt + 1));
-        uint32_t nab[2];
-        uint64_t s[2];
-        SGPB_TRY(read_u32(C, cnt, nab, 2));
-        SGPB_TRY(read_u64(C, (const uint64_t *)sums, s, 2));
+        SGPB_TRY(dzero(C, sums, 4 * sizeof(unsigned long long)));
+        SGPB_TRY(avg <= 10 ? gain_pass(G2()) : avg <= 100 ? gain_pass(G8()) : gain_pass(G32()));
+        uint64_t s[4];
+        SGPB_TRY(read_u64(C, (const uint64_t *)sums, s, 4));
         const long long cut0 = (long long)(s[0] / 2), bal0 = (long long)s[1];
         if (pass == 0 && cut_out) *cut_out = (uint64_t)cut0;
-        const uint32_t na = nab[0], nb = nab[1], k = na + nb;
+        const uint32_t na = (uint32_t)s[2], nb = (uint32_t)s[3], k = na + nb;
         C.kernel_launches += 1;
         if (k == 0) break;
-        // stable counting sort of each list by descending clamped gain
-        for (int sd = 0; sd < 2; sd++) {
-            const uint32_t len = sd == 0 ? na : nb;
-            if (!len) continue;
-            const uint32_t *src = sd == 0 ? A : B;
-            uint32_t *dst = sd == 0 ? sa : sb;
-            const uint32_t nt = cdiv(len, kFmTile);
-            k_fm_hist<<<nt, kFmTile, 0, C.stream>>>(len, src, gain, nt, hist);
-            SGPB_TRY(scan_u32(C, hist, off, kFmBuckets * nt, nullptr));
-            k_fm_place<<<nt, kFmTile, 0, C.stream>>>(len, src, gain, nt, off, dst);
-            C.kernel_launches += 2;
+        // both sides' candidates in id order, sorted by descending clamped gain
+        if (n < 0x80000000u) {
+            SGPB_TRY(scan_u32(C, flag, pos, 2 * n, nullptr));
+            k_fm_list<<<cdiv(2 * (uint64_t)n, 256), 256, 0, C.stream>>>(2 * n, flag, pos, n, idx);
+        } else {   // one side at a time: 2n does not fit 32 bits
+            for (int sd = 0; sd < 2; sd++) {
+                SGPB_TRY(scan_u32(C, flag + (size_t)sd * n, pos, n, nullptr));
+                k_fm_list<<<cdiv(n, 256), 256, 0, C.stream>>>(n, flag + (size_t)sd * n, pos, n, idx + (sd ? na : 0));
+            }
         }
-        SGPB_CUDA(cudaMemsetAsync(rank, 0xFF, sizeof(uint32_t) * n, C.stream));
+        const uint32_t nt = cdiv(k, kFmTile);
+        if ((uint64_t)kFmKeys * nt > 0xFFFFFFFFull) {
+            set_error("FM: %u vertices of positive gain; their sort holds fewer than 2^31", k);
+            return SGP_B200_ERR_TOO_LARGE;
+        }
+        if (nt > hist_tiles) {
+            SGPB_TRY(dalloc_t(C, &hist, (size_t)kFmKeys * nt + 1));
+            SGPB_TRY(dalloc_t(C, &off, (size_t)kFmKeys * nt + 1));
+            hist_tiles = nt;
+        }
+        k_fm_hist<<<nt, kFmTile, 0, C.stream>>>(k, na, idx, gain, nt, hist);
+        SGPB_TRY(scan_u32(C, hist, off, kFmKeys * nt, nullptr));
+        k_fm_place<<<nt, kFmTile, 0, C.stream>>>(k, na, idx, gain, nt, off, sorted);
+        C.kernel_launches += 3;
+        const uint32_t *sa = sorted, *sb = sorted + na;
+        const unsigned long long key0 = ((unsigned long long)cut0 << 32) | 0xFFFFFFFFull;
+        SGPB_TRY(dzero(C, listed, sizeof(uint32_t) * words));   // ranks are read of listed vertices alone
         k_fm_interleave<<<fm_grid(C, na > nb ? na : nb), 256, 0, C.stream>>>(na, nb, sa, sb, gain, bal0, order, rank,
-                                                                             side);
-#define SGPB_FMS(G) k_fm_seqgain<G><<<fm_grid(C, (uint64_t)k * G), 256, 0, C.stream>>>(k, L.rp, L.col, part, order, rank, gseq)
-        if (avg <= 4) SGPB_FMS(4);
-        else if (avg <= 16) SGPB_FMS(16);
-        else SGPB_FMS(32);
-#undef SGPB_FMS
+                                                                             listed, side, key0, best);
+        SGPB_TRY(avg <= 10 ? seq_pass(G2(), k) : avg <= 100 ? seq_pass(G8(), k) : seq_pass(G32(), k));
         FmBestArgs ba;
         ba.k = k;
         ba.gseq = gseq;
@@ -367,8 +503,6 @@ static int fm_impl(Context &C, const Level &L, const W *w, uint32_t *part, uint3
         ba.chunk_g = chunk_g;
         ba.chunk_b = chunk_b;
         ba.best = best;
-        const unsigned long long key0 = ((unsigned long long)cut0 << 32) | 0xFFFFFFFFull;   // k = 0
-        SGPB_CUDA(cudaMemcpyAsync(best, &key0, sizeof(key0), cudaMemcpyHostToDevice, C.stream));
         uint32_t bg = cdiv(k, 1024);
         if (bg > bgrid_max) bg = bgrid_max;
         if (bg < 1) bg = 1;
@@ -380,7 +514,7 @@ static int fm_impl(Context &C, const Level &L, const W *w, uint32_t *part, uint3
         const uint32_t kstar = 0xFFFFFFFFu - (uint32_t)(bk & 0xFFFFFFFFu);
         const long long best_cut = (long long)(bk >> 32);
         if (kstar == 0 || best_cut == cut0) break;
-        k_fm_apply<<<fm_grid(C, kstar), 256, 0, C.stream>>>(kstar, order, part);
+        k_fm_apply<<<fm_grid(C, kstar), 256, 0, C.stream>>>(kstar, order, part, bits);
         C.kernel_launches++;
         SGPB_CUDA(cudaGetLastError());
         moves += kstar;

@@ -217,6 +217,10 @@ int power_iter_mid_chains(Context &C, const std::vector<PIChain *> &chains, cons
 int split_level(Context &C, const Level &L, const double *evec, int perc_imbalance, uint32_t *part,
                 uint64_t *edgecut, uint32_t *n_part0);
 int edge_cut_device(Context &C, const Level &L, const uint32_t *part, uint64_t *edgecut);
+// bitmap of a part array (bits.cuh); the rows of more than kLongRow entries in
+// any order, their number added to *nlong
+int part_bits(Context &C, uint32_t n, const uint32_t *part, uint32_t *bits);
+int long_rows(Context &C, uint32_t n, const uint32_t *rp, uint32_t *longs, uint32_t *nlong);
 // the reference's local search after the split (sgpar.h:2080-2170); mid =
 // the part-0 size the split left
 int local_search_level(Context &C, const Level &L, uint32_t *part, uint32_t mid, uint32_t *swaps_out,

@@ -6,23 +6,34 @@
 // while that does not raise the cut; edge cut = directed cross entries / 2.
 //
 // The reference sorts all n pairs on the host.  Only the order statistic at
-// position imbl matters for the split, so this is a radix *select*: twelve
-// 8-bit digit passes (64 key bits of the order-preserving image of the double,
-// then 32 index bits) inside one cooperative kernel, each pass a histogram
-// and a grid barrier.  part[i] = ((key_i, i) < threshold) ? 0 : 1, then one
-// pass over the CSR counts the cut and the single sweep vertex of an odd n
+// position imbl matters for the split, so this is a radix *select* over the 64
+// key bits of the order-preserving image of the double, then the 32 index
+// bits, in one cooperative kernel: 11 bits a pass, each pass a histogram and a
+// grid barrier, until at most kSelSmall candidates are left, which every
+// block ranks for itself.  part[i] = ((key_i, i) < threshold) ? 0 : 1, also as
+// a bitmap.  A pass over the CSR then counts the cut from the bitmap in
+// shared memory, and the single sweep vertex of an odd n
 // (perc_imbalance_allowed = 0, the value the reference's driver passes,
 // sgpar.cpp:55) is decided on the device.
+//
+// What bounds it: the select is a chain of grid barriers (three or four where
+// the 12 digit passes of 8 bits took 13), the cut the row lookups of short
+// rows and the destination stream.  Erdos-Renyi, 1M vertices, 8M entries: 380
+// -> 80 us.
 #include <mutex>
 
 #include <cooperative_groups.h>
 
+#include "bits.cuh"
 #include "common.cuh"
 #include "internal.h"
 
 namespace sgpb {
 
 constexpr int kSplitThreads = 512;
+
+constexpr int kSelBits = 11, kSelBins = 1 << kSelBits;
+constexpr uint32_t kSelSmall = 1024;       // candidates ranked directly
 
 struct SplitArgs {
     uint32_t n;
@@ -31,12 +42,14 @@ struct SplitArgs {
     const double *evec;
     uint32_t k;            // imbl: sorted position of the threshold element
     uint32_t sweep;        // 1 when position k is also the sweep vertex (imbr - imbl == 1)
-    unsigned long long *keys;
-    uint32_t *hist;        // [3][256], all zero at launch
+    uint32_t *hist;        // [3][kSelBins], then the candidate and the long-row counter: all zero at launch
+    unsigned long long *cand;       // [2 * kSelSmall] (key, index) of the last candidates
+    uint32_t *bits;        // [bit_words(n)] part 1
+    uint32_t *longs;       // rows of more than kLongRow entries, in any order
     uint32_t *part;
-    unsigned long long *cut_part;   // [gridDim]
-    unsigned long long *out;        // [0] edgecut [1] part0 size [2] threshold index
+    unsigned long long *out;        // [0] edgecut [1] part0 size [2] threshold index [3] directed cross entries
 };
+constexpr size_t kSplitHistWords = 3 * kSelBins + 2;
 
 __device__ __forceinline__ unsigned long long order_key(double x) {
     if (x == 0.0) x = 0.0;   // -0.0 == +0.0 in the reference's comparator
@@ -46,136 +59,261 @@ __device__ __forceinline__ unsigned long long order_key(double x) {
 
 __global__ void __launch_bounds__(kSplitThreads) k_split(SplitArgs a) {
     cg::grid_group grid = cg::this_grid();
-    __shared__ uint32_t sh[256];
+    __shared__ uint32_t sh[kSelBins];
     __shared__ uint64_t sm[64];
+    __shared__ unsigned long long s_key[kSelSmall];
+    __shared__ uint32_t s_idx[kSelSmall];
+    __shared__ uint32_t s_sel[3];
     const uint32_t n = a.n;
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = tid; i < n; i += nth) a.keys[i] = order_key(a.evec[i]);
-    // select: prefix over (key:64, index:32) = 96 bits, 12 digits MSB first
+    uint32_t *ncand = a.hist + 3 * kSelBins, *nlong = ncand + 1;
+    // select: prefix over (key:64, index:32), digits MSB first: the key in five
+    // of 11 bits and one of 9, the index in two of 11 and one of 10
     unsigned long long kpre = 0;   // selected key bits so far
     uint32_t ipre = 0;             // selected index bits so far
     uint32_t rank = a.k;           // rank among candidates matching the prefix
-    for (int pass = 0; pass < 12; pass++) {
-        uint32_t *h = a.hist + (pass % 3) * 256;
+    for (int pass = 0; pass < 9; pass++) {
+        uint32_t *h = a.hist + (pass % 3) * kSelBins;
         // Clear the buffer of the next pass.  It was last read after the barrier
         // of pass - 2, which every block has passed; it is next written after the
         // barrier of this pass.
-        if (blockIdx.x == 0)
-            for (int t = threadIdx.x; t < 256; t += blockDim.x) a.hist[((pass + 1) % 3) * 256 + t] = 0;
-        for (int t = threadIdx.x; t < 256; t += blockDim.x) sh[t] = 0;
+        if (blockIdx.x == 0 && pass > 0)
+            for (int t = threadIdx.x; t < kSelBins; t += blockDim.x) a.hist[((pass + 1) % 3) * kSelBins + t] = 0;
+        for (int t = threadIdx.x; t < kSelBins; t += blockDim.x) sh[t] = 0;
         __syncthreads();
+        const bool by_key = pass < 6;
+        const int shift = by_key ? (pass < 5 ? 53 - 11 * pass : 0) : (pass < 8 ? 21 - 11 * (pass - 6) : 0);
+        const uint32_t width = by_key ? (pass < 5 ? 11u : 9u) : (pass < 8 ? 11u : 10u), mask = (1u << width) - 1u;
         for (uint64_t i = tid; i < n; i += nth) {
-            unsigned long long key = a.keys[i];
+            const unsigned long long key = order_key(a.evec[i]);
             uint32_t digit;
-            if (pass < 8) {
-                int shift = 56 - 8 * pass;
+            if (by_key) {
                 // candidates: key bits above the current digit equal the prefix
-                unsigned long long hi = pass == 0 ? 0 : (key >> (shift + 8));
-                unsigned long long phi = pass == 0 ? 0 : (kpre >> (shift + 8));
-                if (hi != phi) continue;
-                digit = (uint32_t)((key >> shift) & 0xFF);
+                if (pass && (key >> (shift + width)) != (kpre >> (shift + width))) continue;
+                digit = (uint32_t)(key >> shift) & mask;
             } else {
                 if (key != kpre) continue;
-                int shift = 24 - 8 * (pass - 8);
-                uint32_t idx = (uint32_t)i;
-                uint32_t hi = pass == 8 ? 0 : (idx >> (shift + 8));
-                uint32_t phi = pass == 8 ? 0 : (ipre >> (shift + 8));
-                if (hi != phi) continue;
-                digit = (idx >> shift) & 0xFF;
+                if (pass > 6 && ((uint32_t)i >> (shift + width)) != (ipre >> (shift + width))) continue;
+                digit = ((uint32_t)i >> shift) & mask;
             }
             atomicAdd(&sh[digit], 1u);
         }
+        if (pass == 0)   // beside the first pass: the rows the cut gives to whole blocks
+            for (uint64_t i = tid; i < n; i += nth)
+                if (a.rp[i + 1] - a.rp[i] > kLongRow) a.longs[atomicAdd(nlong, 1u)] = (uint32_t)i;
         __syncthreads();
-        for (int t = threadIdx.x; t < 256; t += blockDim.x)
+        for (int t = threadIdx.x; t < kSelBins; t += blockDim.x)
             if (sh[t]) atomicAdd(&h[t], sh[t]);
         grid.sync();
         // every block picks the same digit from the global histogram
-        if (threadIdx.x == 0) {
-            uint32_t acc = 0, d = 0;
-            for (d = 0; d < 256; d++) {
-                uint32_t c = h[d];
-                if (rank < acc + c) break;
-                acc += c;
+        {
+            constexpr int per = kSelBins / kSplitThreads;
+            uint32_t c[per];
+            uint64_t sum = 0, tot;
+#pragma unroll
+            for (int q = 0; q < per; q++) {
+                c[q] = __ldcg(h + threadIdx.x * per + q);
+                sum += c[q];
             }
-            sh[0] = d;
-            sh[1] = rank - acc;
-        }
-        __syncthreads();
-        const uint32_t d = sh[0];
-        rank = sh[1];
-        if (pass < 8) kpre |= (unsigned long long)d << (56 - 8 * pass);
-        else ipre |= d << (24 - 8 * (pass - 8));
-        __syncthreads();
-    }
-    // assign parts
-    uint64_t c0 = 0;
-    for (uint64_t i = tid; i < n; i += nth) {
-        unsigned long long key = a.keys[i];
-        bool less = key < kpre || (key == kpre && (uint32_t)i < ipre);
-        a.part[i] = less ? 0u : 1u;
-        c0 += less;
-    }
-    grid.sync();
-    // directed cross entries, one warp per row
-    uint64_t cut = 0;
-    {
-        const unsigned lane = threadIdx.x & 31;
-        const uint64_t wid = tid >> 5, nw = nth >> 5;
-        for (uint64_t i = wid; i < n; i += nw) {
-            const uint32_t pi = a.part[i];
-            uint32_t c = 0;
-            for (uint32_t j = a.rp[i] + lane; j < a.rp[i + 1]; j += 32) c += (a.part[a.col[j]] != pi);
-            cut += c;
-        }
-    }
-    {
-        uint64_t t1, t2;
-        block_scan_u64(cut, sm, &t1);
-        block_scan_u64(c0, sm, &t2);
-        if (threadIdx.x == 0) {
-            a.cut_part[2 * blockIdx.x] = t1;
-            a.cut_part[2 * blockIdx.x + 1] = t2;
-        }
-    }
-    grid.sync();
-    if (blockIdx.x == 0) {
-        uint64_t s = 0, s0 = 0;
-        for (uint32_t b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
-            s += a.cut_part[2 * b];
-            s0 += a.cut_part[2 * b + 1];
-        }
-        uint64_t tot, tot0;
-        block_scan_u64(s, sm, &tot);
-        block_scan_u64(s0, sm, &tot0);
-        // sweep of the vertex at position k (sgpar.h:2046-2071)
-        long long upd = 0;
-        if (a.sweep) {
-            const uint32_t u = ipre;
-            long long c = 0;
-            for (uint32_t j = a.rp[u] + threadIdx.x; j < a.rp[u + 1]; j += blockDim.x)
-                c += (a.part[a.col[j]] == 1) ? 1 : -1;
-            uint64_t uc = (uint64_t)(c + (1ll << 40));   // bias to keep the scan unsigned
-            uint64_t tt;
-            block_scan_u64(uc, sm, &tt);
-            upd = (long long)tt - (long long)blockDim.x * (1ll << 40);
-        }
-        if (threadIdx.x == 0) {
-            long long cur = (long long)tot, best = (long long)tot;
-            uint64_t p0 = tot0;
-            if (a.sweep) {
-                cur = cur + 2 * upd;
-                if (cur <= best) {
-                    a.part[ipre] = 0;
-                    best = cur;
-                    p0++;
+            uint64_t acc = block_scan_u64(sum, sm, &tot) - sum;
+#pragma unroll
+            for (int q = 0; q < per; q++) {
+                if (rank >= acc && rank < acc + c[q]) {
+                    s_sel[0] = threadIdx.x * per + q;
+                    s_sel[1] = rank - (uint32_t)acc;
+                    s_sel[2] = c[q];
                 }
+                acc += c[q];
             }
-            a.out[0] = (unsigned long long)(best / 2);
-            a.out[1] = p0;
-            a.out[2] = ipre;
         }
+        __syncthreads();
+        const uint32_t d = s_sel[0], left = s_sel[2];
+        rank = s_sel[1];
+        if (by_key) kpre |= (unsigned long long)d << shift;
+        else ipre |= d << shift;
+        __syncthreads();
+        if (pass == 8) break;
+        if (left > kSelSmall) continue;
+        // few enough: list them, and every block ranks the list
+        for (uint64_t i = tid; i < n; i += nth) {
+            const unsigned long long key = order_key(a.evec[i]);
+            const bool in = by_key ? (key >> shift) == (kpre >> shift)
+                                   : key == kpre && ((uint32_t)i >> shift) == (ipre >> shift);
+            if (in) {
+                const uint32_t q = atomicAdd(ncand, 1u);
+                a.cand[2 * q] = key;
+                a.cand[2 * q + 1] = i;
+            }
+        }
+        grid.sync();
+        for (uint32_t q = threadIdx.x; q < left; q += blockDim.x) {
+            s_key[q] = __ldcg(a.cand + 2 * q);
+            s_idx[q] = (uint32_t)__ldcg(a.cand + 2 * q + 1);
+        }
+        __syncthreads();
+        for (uint32_t q = threadIdx.x; q < left; q += blockDim.x) {
+            const unsigned long long key = s_key[q];
+            const uint32_t idx = s_idx[q];
+            uint32_t before = 0;
+            for (uint32_t t = 0; t < left; t++) before += s_key[t] < key || (s_key[t] == key && s_idx[t] < idx);
+            if (before == rank) {   // one entry of the list: no two are equal
+                sm[40] = key;
+                s_sel[0] = idx;
+            }
+        }
+        __syncthreads();
+        kpre = sm[40];
+        ipre = s_sel[0];
+        break;
     }
+    // assign parts; a.k elements precede the threshold
+    for (uint64_t i0 = tid & ~31ull; i0 < n; i0 += nth) {
+        const uint64_t i = i0 + (threadIdx.x & 31);
+        bool less = true;
+        if (i < n) {
+            const unsigned long long key = order_key(a.evec[i]);
+            less = key < kpre || (key == kpre && (uint32_t)i < ipre);
+            a.part[i] = less ? 0u : 1u;
+        }
+        const unsigned b = __ballot_sync(0xFFFFFFFFu, !less);
+        if ((threadIdx.x & 31) == 0) a.bits[i0 >> 5] = b;
+    }
+    if (tid == 0) {
+        a.out[1] = a.k;
+        a.out[2] = ipre;
+        a.out[3] = 0;
+    }
+}
+
+// the bitmap of a part array
+__global__ void k_part_bits(uint32_t n, const uint32_t *__restrict__ part, uint32_t *__restrict__ bits) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned b = __ballot_sync(0xFFFFFFFFu, i < n && part[i] != 0);
+    if ((threadIdx.x & 31) == 0 && i < n) bits[i >> 5] = b;
+}
+
+__global__ void k_long_rows(uint32_t n, const uint32_t *__restrict__ rp, uint32_t *__restrict__ longs,
+                            uint32_t *__restrict__ nlong) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n && rp[i + 1] - rp[i] > kLongRow) longs[atomicAdd(nlong, 1u)] = i;
+}
+
+// Cross entries of rows of at most kLongRow entries, G lanes a row and four
+// entries a lane in flight.
+template <int G>
+__device__ __forceinline__ uint64_t cut_rows(uint32_t n, const uint32_t *__restrict__ rp,
+                                             const uint32_t *__restrict__ col, const uint32_t *bits) {
+    const uint32_t lane = threadIdx.x & (G - 1);
+    const uint64_t ng = ((uint64_t)gridDim.x * blockDim.x) / G;
+    uint64_t cut = 0;
+    for (uint64_t u = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / G; u < n; u += ng) {
+        const uint32_t b = __ldg(rp + u), e = __ldg(rp + u + 1);
+        if (e - b > kLongRow) continue;
+        const uint32_t pu = bit_of(bits, (uint32_t)u);
+        uint32_t c = 0;
+        for (uint32_t j0 = b + lane; j0 < e; j0 += 4 * G) {
+            uint32_t v[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) v[q] = j0 + q * G < e ? __ldg(col + j0 + q * G) : (uint32_t)u;
+#pragma unroll
+            for (int q = 0; q < 4; q++) c += bit_of(bits, v[q]) != pu;
+        }
+        cut += c;
+    }
+    return cut;
+}
+
+// Directed cross entries of a bisection given as a bitmap, added to *out.
+// SHARED: the bitmap in the block's shared memory.
+template <bool SHARED>
+__global__ void __launch_bounds__(1024) k_cut_bits(uint32_t n, const uint32_t *__restrict__ rp,
+                                                   const uint32_t *__restrict__ col, const uint32_t *__restrict__ gbits,
+                                                   const uint32_t *__restrict__ longs,
+                                                   const uint32_t *__restrict__ nlong, unsigned long long *out) {
+    extern __shared__ uint32_t s_bits[];
+    __shared__ uint64_t sm[33];
+    const uint32_t m = __ldg(rp + n);
+    if (SHARED) {
+        bits_load(gbits, bit_words(n), s_bits);
+        __syncthreads();
+    }
+    const uint32_t *bits = SHARED ? (const uint32_t *)s_bits : gbits;
+    uint64_t cut;
+    // a row's latency is what short rows cost: lanes for about a trip a row
+    if (m <= 10ull * n) cut = cut_rows<2>(n, rp, col, bits);
+    else if (m <= 20ull * n) cut = cut_rows<4>(n, rp, col, bits);
+    else if (m <= 100ull * n) cut = cut_rows<8>(n, rp, col, bits);
+    else cut = cut_rows<32>(n, rp, col, bits);
+    // long rows, a block each
+    const uint32_t nl = *nlong;
+    for (uint32_t r = blockIdx.x; r < nl; r += gridDim.x) {
+        const uint32_t u = __ldg(longs + r), b = __ldg(rp + u), e = __ldg(rp + u + 1);
+        const uint32_t pu = bit_of(bits, u);
+#pragma unroll 4
+        for (uint64_t j = (uint64_t)b + threadIdx.x; j < e; j += 1024) cut += bit_of(bits, __ldg(col + j)) != pu;
+    }
+    uint64_t tot;
+    block_scan_u64(cut, sm, &tot);
+    if (threadIdx.x == 0 && tot) atomicAdd(out, (unsigned long long)tot);
+}
+
+// sweep of the vertex at position k (sgpar.h:2046-2071) and the results
+__global__ void __launch_bounds__(kSplitThreads) k_split_sweep(SplitArgs a) {
+    __shared__ uint64_t sm[64];
+    long long upd = 0;
+    const uint32_t u = (uint32_t)a.out[2];
+    if (a.sweep) {
+        long long c = 0;
+        for (uint32_t j = a.rp[u] + threadIdx.x; j < a.rp[u + 1]; j += blockDim.x)
+            c += (a.part[a.col[j]] == 1) ? 1 : -1;
+        uint64_t uc = (uint64_t)(c + (1ll << 40));   // bias to keep the scan unsigned
+        uint64_t tt;
+        block_scan_u64(uc, sm, &tt);
+        upd = (long long)tt - (long long)blockDim.x * (1ll << 40);
+    }
+    if (threadIdx.x == 0) {
+        long long best = (long long)a.out[3];
+        if (a.sweep) {
+            const long long cur = best + 2 * upd;
+            if (cur <= best) {
+                a.part[u] = 0;
+                best = cur;
+                a.out[1]++;
+            }
+        }
+        a.out[0] = (unsigned long long)(best / 2);
+    }
+}
+
+static int launch_cut_bits(cudaStream_t s, int num_sms, uint32_t n, const uint32_t *rp, const uint32_t *col,
+                           const uint32_t *bits, const uint32_t *longs, const uint32_t *nlong,
+                           unsigned long long *out) {
+    const uint32_t words = bit_words(n);
+    const size_t bytes = (size_t)words * 4;
+    // two blocks an SM while two bitmaps fit; a block per 4096 rows at least
+    uint32_t g = (uint32_t)num_sms * (words <= kBitsMaxWords / 2 || words > kBitsMaxWords ? 2u : 1u);
+    if (g > cdiv(n, 256)) g = cdiv(n, 256);
+    if (words <= kBitsMaxWords) {
+        SGPB_CUDA(cudaFuncSetAttribute(k_cut_bits<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(kBitsMaxWords * 4)));
+        k_cut_bits<true><<<g, 1024, bytes, s>>>(n, rp, col, bits, longs, nlong, out);
+    } else {
+        k_cut_bits<false><<<g, 1024, 0, s>>>(n, rp, col, bits, longs, nlong, out);
+    }
+    SGPB_CUDA(cudaGetLastError());
+    return SGP_B200_OK;
+}
+
+// the kernels of a split whose SplitArgs are complete and whose histogram
+// words are zero
+static int launch_split(cudaStream_t s, int num_sms, uint32_t grid, SplitArgs &a) {
+    void *args[] = {&a};
+    SGPB_CUDA(cudaLaunchCooperativeKernel((const void *)k_split, dim3(grid), dim3(kSplitThreads), args, 0, s));
+    SGPB_TRY(launch_cut_bits(s, num_sms, a.n, a.rp, a.col, a.bits, a.longs, a.hist + 3 * kSelBins + 1, a.out + 3));
+    k_split_sweep<<<1, kSplitThreads, 0, s>>>(a);
+    SGPB_CUDA(cudaGetLastError());
+    return SGP_B200_OK;
 }
 
 int split_level(Context &C, const Level &L, const double *evec, int perc_imbalance, uint32_t *part,
@@ -195,9 +333,11 @@ int split_level(Context &C, const Level &L, const double *evec, int perc_imbalan
     // With imbl == n there is no threshold element (cannot happen for p = 0).
     a.k = imbl < n ? imbl : n - 1;
     a.sweep = (imbr > imbl) ? 1u : 0u;
-    SGPB_TRY(dalloc_t(C, &a.keys, n));
-    SGPB_TRY(dalloc_t(C, &a.hist, 768));
-    SGPB_TRY(dzero(C, a.hist, 768 * sizeof(uint32_t)));
+    SGPB_TRY(dalloc_t(C, &a.hist, kSplitHistWords));
+    SGPB_TRY(dzero(C, a.hist, kSplitHistWords * sizeof(uint32_t)));
+    SGPB_TRY(dalloc_t(C, &a.cand, 2 * kSelSmall));
+    SGPB_TRY(dalloc_t(C, &a.bits, bit_words(n)));
+    SGPB_TRY(dalloc_t(C, &a.longs, n));
     SGPB_TRY(dalloc_t(C, &a.out, 4));
     int per_sm = 0;
     SGPB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)k_split, kSplitThreads, 0));
@@ -207,10 +347,8 @@ int split_level(Context &C, const Level &L, const double *evec, int perc_imbalan
     uint64_t want = cdiv(n, kSplitThreads * 8ull);
     uint32_t grid = (uint32_t)(want < maxg ? want : maxg);
     if (grid < 1) grid = 1;
-    SGPB_TRY(dalloc_t(C, &a.cut_part, 2 * (size_t)grid));
-    void *args[] = {&a};
-    SGPB_CUDA(cudaLaunchCooperativeKernel((const void *)k_split, dim3(grid), dim3(kSplitThreads), args, 0, C.stream));
-    C.kernel_launches++;
+    SGPB_TRY(launch_split(C.stream, C.num_sms, grid, a));
+    C.kernel_launches += 3;
     uint64_t out[3];
     SGPB_TRY(read_u64(C, (const uint64_t *)a.out, out, 3));
     *edgecut = out[0];
@@ -219,17 +357,17 @@ int split_level(Context &C, const Level &L, const double *evec, int perc_imbalan
 }
 
 // --------------------------------------------------- split, no allocation --
-// Scratch of sgp_b200_split_noalloc: sort keys for SGP_B200_NOALLOC_MAX_N
-// vertices, the three digit histograms, per-block cut partials for up to
-// kNoAllocMaxBlocks blocks and the result words.  It is a file-scope device
-// array, so every GPU that loads this library holds it (about 8 MiB) until the
-// process exits, and every call on a device shares it.
+// Scratch of sgp_b200_split_noalloc: the long-row list and the bitmap of
+// SGP_B200_NOALLOC_MAX_N vertices, the last candidates, the digit histograms
+// and the result words.  It is a file-scope device array, so every GPU that
+// loads this library holds it (about 4 MiB) until the process exits, and every
+// call on a device shares it.
 constexpr uint32_t kNoAllocMaxBlocks = 1024;
-constexpr size_t kNoAllocKeysBytes = (size_t)SGP_B200_NOALLOC_MAX_N * sizeof(unsigned long long);
-constexpr size_t kNoAllocHistOff = kNoAllocKeysBytes;
-constexpr size_t kNoAllocCutOff = kNoAllocHistOff + 768 * sizeof(uint32_t);
-constexpr size_t kNoAllocOutOff = kNoAllocCutOff + 2 * (size_t)kNoAllocMaxBlocks * sizeof(unsigned long long);
-constexpr size_t kNoAllocBytes = kNoAllocOutOff + 4 * sizeof(unsigned long long);
+constexpr size_t kNoAllocBitsOff = (size_t)SGP_B200_NOALLOC_MAX_N * sizeof(uint32_t);
+constexpr size_t kNoAllocCandOff = kNoAllocBitsOff + (size_t)SGP_B200_NOALLOC_MAX_N / 8;
+constexpr size_t kNoAllocOutOff = kNoAllocCandOff + 2 * (size_t)kSelSmall * sizeof(unsigned long long);
+constexpr size_t kNoAllocHistOff = kNoAllocOutOff + 4 * sizeof(unsigned long long);
+constexpr size_t kNoAllocBytes = kNoAllocHistOff + kSplitHistWords * sizeof(uint32_t);
 static __device__ __align__(256) unsigned char g_split_scratch[kNoAllocBytes];
 
 // Per-device set-up, done by the first call on that device: the host
@@ -310,28 +448,31 @@ static int noalloc_setup(int device, NoAllocDevice **out) {
 }
 
 // ------------------------------------------------------------- edge cut --
-__global__ void k_cut(uint32_t n, const uint32_t *rp, const uint32_t *col, const uint32_t *part,
-                      unsigned long long *out) {
-    const unsigned lane = threadIdx.x & 31;
-    const uint64_t wid = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    uint32_t c = 0;
-    for (uint64_t i = wid; i < n; i += nw) {
-        const uint32_t pi = part[i];
-        for (uint32_t j = rp[i] + lane; j < rp[i + 1]; j += 32) c += (part[col[j]] != pi);
-    }
-    c = warp_sum(c);
-    if (lane == 0 && c) atomicAdd(out, (unsigned long long)c);
+int part_bits(Context &C, uint32_t n, const uint32_t *part, uint32_t *bits) {
+    k_part_bits<<<cdiv(n, 256), 256, 0, C.stream>>>(n, part, bits);
+    C.kernel_launches++;
+    SGPB_CUDA(cudaGetLastError());
+    return SGP_B200_OK;
+}
+
+int long_rows(Context &C, uint32_t n, const uint32_t *rp, uint32_t *longs, uint32_t *nlong) {
+    k_long_rows<<<cdiv(n, 256), 256, 0, C.stream>>>(n, rp, longs, nlong);
+    C.kernel_launches++;
+    SGPB_CUDA(cudaGetLastError());
+    return SGP_B200_OK;
 }
 
 int edge_cut_device(Context &C, const Level &L, const uint32_t *part, uint64_t *edgecut) {
     unsigned long long *o;
-    SGPB_TRY(dalloc_t(C, &o, 1));
-    SGPB_TRY(dzero(C, o, 8));
+    SGPB_TRY(dalloc_t(C, &o, 2));
+    SGPB_TRY(dzero(C, o, 16));
     if (L.n) {
-        uint32_t g = cdiv(L.n, 8);
-        if (g > (uint32_t)C.num_sms * 8) g = C.num_sms * 8;
-        k_cut<<<g, 256, 0, C.stream>>>(L.n, L.rp, L.col, part, o);
+        uint32_t *bits, *longs, *nlong = (uint32_t *)(o + 1);
+        SGPB_TRY(dalloc_t(C, &bits, bit_words(L.n)));
+        SGPB_TRY(dalloc_t(C, &longs, L.n));
+        SGPB_TRY(part_bits(C, L.n, part, bits));
+        SGPB_TRY(long_rows(C, L.n, L.rp, longs, nlong));
+        SGPB_TRY(launch_cut_bits(C.stream, C.num_sms, L.n, L.rp, L.col, bits, longs, nlong, o));
         C.kernel_launches++;
     }
     uint64_t h;
@@ -635,21 +776,21 @@ extern "C" int sgp_b200_split_noalloc(void *stream, uint32_t n, const uint32_t *
     const uint32_t imbl = n - imbr;
     a.k = imbl < n ? imbl : n - 1;
     a.sweep = imbr > imbl ? 1u : 0u;
-    a.keys = reinterpret_cast<unsigned long long *>(d->scratch);
+    a.longs = reinterpret_cast<uint32_t *>(d->scratch);
+    a.bits = reinterpret_cast<uint32_t *>(d->scratch + kNoAllocBitsOff);
+    a.cand = reinterpret_cast<unsigned long long *>(d->scratch + kNoAllocCandOff);
     a.hist = reinterpret_cast<uint32_t *>(d->scratch + kNoAllocHistOff);
-    a.cut_part = reinterpret_cast<unsigned long long *>(d->scratch + kNoAllocCutOff);
     a.out = reinterpret_cast<unsigned long long *>(d->scratch + kNoAllocOutOff);
-    // the scratch keeps the previous call's contents: the histograms must
-    // start at zero; keys, partials and results are written before use
-    SGPB_CUDA(cudaMemsetAsync(a.hist, 0, 768 * sizeof(uint32_t), s));
+    // the scratch keeps the previous call's contents: the histograms and
+    // counters must start at zero; the rest is written before use
+    SGPB_CUDA(cudaMemsetAsync(a.hist, 0, kSplitHistWords * sizeof(uint32_t), s));
     const int per_sm = d->per_sm > 2 ? 2 : d->per_sm;
     uint64_t grid = (uint64_t)per_sm * d->num_sms;
     const uint64_t want = cdiv(n, kSplitThreads * 8ull);
     if (want < grid) grid = want;
     if (grid > kNoAllocMaxBlocks) grid = kNoAllocMaxBlocks;
     if (grid < 1) grid = 1;
-    void *args[] = {&a};
-    SGPB_CUDA(cudaLaunchCooperativeKernel((const void *)k_split, dim3((unsigned)grid), dim3(kSplitThreads), args, 0, s));
+    SGPB_TRY(launch_split(s, d->num_sms, (uint32_t)grid, a));
     // result[0] = edge cut, result[1] = size of part 0 (device array)
     SGPB_CUDA(cudaMemcpyAsync(result, a.out, 2 * sizeof(uint64_t), cudaMemcpyDeviceToDevice, s));
     SGPB_CUDA(cudaGetLastError());
