@@ -8,7 +8,7 @@
 // entries; rows above 32 * epl entries are cut into units of that size.  Rows
 // are summed by their lanes in entry order and combined by a butterfly.
 //
-// Three forms, chosen per level (slice_form):
+// Four forms, chosen per level (slice_form):
 //   direct, shared   the whole iterate in every block's shared memory
 //                    (n <= kSlicePW), one grid barrier an iteration
 //   panels           columns cut into panels of kSlicePW; a block loads the
@@ -17,6 +17,8 @@
 //                    barrier the rows add their panels
 //   direct, global   iterate gathered from L2 (sparse levels wider than one
 //                    panel), one grid barrier an iteration
+//   direct, hub      the same in degree order, the leading kSlicePW entries (the
+//                    most referenced) in shared memory (skewed levels)
 // Destinations are 16 bits inside a panel, weights 8 / 16 / 32 / 64 bits, or
 // none: a level whose total weight is at most 1.25 times its entries repeats
 // them instead (first coarse levels of unweighted graphs: 1.09 at R-MAT 22).
@@ -26,11 +28,13 @@
 // half warp's 64-bit gathers in one pass when its 16 banks differ: 6.4 passes
 // a warp load with the entries in row order, 3.0 with the places chosen by
 // bank (R-MAT 20's first coarse level, 30.6M entries).  An iteration of R-MAT
-// 22's level 1 (117M entries) goes from 341 us to 123, of R-MAT 20's from 96
-// to 39, of a weighted Chung-Lu level of 5.9M entries from 49 to 20, of a mesh
-// level of 16,799 vertices from 11.1 to 5.9.  What is left is the 2-byte
-// matrix stream (about 50 us of the 123) and, below a million entries, the
-// barrier and the trips to L2 behind it (about 4 us an iteration).
+// 22's level 1 (117M entries) goes from 341 us to 116, of R-MAT 20's from 96
+// to 37, of a weighted Chung-Lu level of 5.9M entries from 49 to 20, of a mesh
+// level of 16,799 vertices from 11.1 to 5.9, of one of 190,000 from 26 to 10.5.
+// What is left is the shared-memory passes (49 us of the 116) and the 2-byte
+// matrix stream (47 us) overlapped with them, the rows' panel sums (15 us) and,
+// below a million entries, the barrier and the trips to L2 behind it (about 4
+// us an iteration).
 //
 // Sums are taken in an order fixed by the level and the grid (static unit
 // ranges per warp), so results are reproducible run to run.
@@ -51,18 +55,20 @@ constexpr uint32_t kSlicePW = 25600;        // iterate entries per panel (200 KB
 // destination of an empty place is a zero behind the panel in that bank.
 constexpr uint32_t kBanks = 16;
 constexpr size_t kSliceSmem = (size_t)(kSlicePW + kBanks) * sizeof(double);
-// 512 threads leave each 128 registers for the batches in flight: against
-// 1024 threads the weighted Chung-Lu partition takes 70 instead of 78 ms and
-// R-MAT 16 22 instead of 25 (R-MAT 22's level 1 123 against 118 us an
-// iteration)
-constexpr int kSliceThreads = 512;
-constexpr int kSliceWarps = kSliceThreads / 32;
+enum SliceForm { kFormShared = 0, kFormGlobal = 1, kFormPanels = 2, kFormHub = 3 };
+
+// Threads of a block.  512 leave each 128 registers for the batches in flight:
+// against 1024 threads the weighted Chung-Lu partition takes 70 instead of 78
+// ms and R-MAT 16 22 instead of 25.  Panels without weights hold no weights in
+// registers and gain from the warps instead (R-MAT 22's level 1 125 -> 122 us).
+__host__ __device__ constexpr int slice_threads(int form, int wb) {
+    return form == kFormPanels && wb == 0 ? 1024 : 512;
+}
 constexpr uint32_t kSliceItem = 2048;       // entries of a row that one warp lays out
-constexpr uint32_t kSliceMaxPanels = 32;    // a lane holds a panel's counter while counting
+constexpr uint32_t kSliceMaxPanels = 32;    // a lane holds a panel's bounds in the layout kernels
 constexpr int kSumK = 3;                    // sum r, sum r^2, sum u r
 constexpr uint32_t kSpinLimit = 1u << 28;   // polls of a grid barrier before giving up
 
-enum SliceForm { kFormNone = -1, kFormShared = 0, kFormGlobal = 1, kFormPanels = 2 };
 
 struct SliceArgs {
     uint32_t n, n32, P;
@@ -129,13 +135,14 @@ struct GridBar {
 };
 
 // The block's sums of p[3], written to dst[0..2] by warp 0 (sm: 3 x 32).
+template <int WARPS>
 __device__ __forceinline__ void block_sum3_to(const double (&p)[kSumK], double (*sm)[kSumK], double *dst) {
     const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const double v = warp_sum3(p[0], p[1], p[2]);
     if (lane < kSumK) sm[wid][lane] = v;
     __syncthreads();
     if (wid == 0) {
-        const bool in = lane < kSliceWarps;
+        const bool in = lane < WARPS;
         const double t = warp_sum3(in ? sm[lane][0] : 0.0, in ? sm[lane][1] : 0.0, in ? sm[lane][2] : 0.0);
         if (lane < kSumK) dst[lane] = t;
     }
@@ -218,14 +225,15 @@ struct Wgt4 {
 // destinations and weights are one stream, loaded a batch of U steps ahead of
 // its use across unit ends.  begin() loads the first batch (it depends on the
 // layout alone, so a barrier can follow); run() consumes the stream and calls
-// done(unit, next unit, sum) on every lane at each unit's end (the sum complete on all
+// done(unit, next unit, whether there is one, sum) on every lane at each unit's end (the sum complete on all
 // lanes of a row).
-template <bool GLOBAL, bool PANELS, int WB>
+template <int FORM, int WB>
 struct Stream {
+    static constexpr bool GLOBAL = FORM == kFormGlobal || FORM == kFormHub, PANELS = FORM == kFormPanels;
     typedef typename std::conditional<GLOBAL, Col32, Col16>::type Col;
-    static constexpr int U = (GLOBAL || WB >= 4) ? 2 : (PANELS && WB == 0) ? 8 : 4;
+    static constexpr int U = (GLOBAL || WB >= 4) ? 2 : 4;
     uint32_t k, k1, pos, end;   // unit, last unit's end, stream position and end in steps
-    uint4 d, dn;                // this unit's record and the next one's
+    uint4 d, dn, dm;            // records of this unit and of the next two
     Col c[U];
     Wgt4<WB> w[U];
 
@@ -236,6 +244,7 @@ struct Stream {
         if (k >= k1) return;
         d = __ldg(a.unit + k);
         dn = __ldg(a.unit + (k + 1 < k1 ? k + 1 : k));
+        dm = __ldg(a.unit + (k + 2 < k1 ? k + 2 : k));
         const uint4 dl = __ldg(a.unit + k1 - 1);
         pos = d.x;
         end = dl.x + (dl.z & 0xFFFFu);
@@ -251,7 +260,7 @@ struct Stream {
             }
     }
     template <typename Done>
-    __device__ __forceinline__ void run(const SliceArgs &a, const double *x, Done &&done) {
+    __device__ __forceinline__ void run(const SliceArgs &a, const double *x, const double *g, Done &&done) {
         if (k >= k1) return;
         uint32_t left = d.z & 0xFFFFu;
         double s0 = 0, s1 = 0;
@@ -261,11 +270,12 @@ struct Stream {
                 const uint32_t lg = d.z >> 16;
                 double s = s0 + s1;
                 for (uint32_t o = 1; o < (1u << lg); o <<= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-                done(d, dn, s);
+                done(d, dn, k + 1 < k1, s);
                 s0 = s1 = 0;
                 d = dn;
                 k++;
-                if (k + 1 < k1) dn = __ldg(a.unit + k + 1);
+                dn = dm;
+                if (k + 2 < k1) dm = __ldg(a.unit + k + 2);
                 left = d.z & 0xFFFFu;
             } while (left == 0 && k < k1);
         };
@@ -274,7 +284,9 @@ struct Stream {
 #pragma unroll
             for (int e = 0; e < 4; e++) {
                 const uint32_t j = c[q].get(e);
-                if (GLOBAL) v[e] = j != 0xFFFFFFFFu ? x[j] : 0.0;
+                // x: shared memory; g: the whole iterate
+                if (FORM == kFormHub) v[e] = j < kSlicePW ? x[j] : j != 0xFFFFFFFFu ? g[j] : 0.0;
+                else if (GLOBAL) v[e] = j != 0xFFFFFFFFu ? g[j] : 0.0;
                 else v[e] = x[j];
             }
         };
@@ -358,6 +370,7 @@ struct PanelCopy {
 };
 
 // the calling warp's share of the units [u, ue): equal cost
+template <int kSliceWarps>
 __device__ __forceinline__ void warp_units(const SliceArgs &a, uint32_t u, uint32_t ue, unsigned wid, uint32_t &k0,
                                            uint32_t &k1) {
     const uint64_t c0 = a.cpre[u], c1 = a.cpre[ue];
@@ -367,8 +380,10 @@ __device__ __forceinline__ void warp_units(const SliceArgs &a, uint32_t u, uint3
 
 // FORM: the level's form; WB: bytes per weight (0: none).
 template <int FORM, int WB>
-__global__ void __launch_bounds__(kSliceThreads, 1) k_pi_slices(SliceArgs a) {
-    constexpr bool PANELS = FORM == kFormPanels, GLOBAL = FORM == kFormGlobal;
+__global__ void __launch_bounds__(slice_threads(FORM, WB), 1) k_pi_slices(SliceArgs a) {
+    constexpr int kSliceThreads = slice_threads(FORM, WB), kSliceWarps = kSliceThreads / 32;
+    constexpr bool PANELS = FORM == kFormPanels, GLOBAL = FORM == kFormGlobal || FORM == kFormHub;
+    constexpr bool COPY = FORM != kFormGlobal;   // the iterate or a part of it in shared memory
     extern __shared__ __align__(16) double xs[];
     __shared__ double sm[kSliceWarps][kSumK];
     __shared__ double s_sum[4];
@@ -380,9 +395,9 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pi_slices(SliceArgs a) {
     __shared__ __align__(8) uint64_t s_mbar;
     GridBar bar{a.bar, a.err, 0};
     PanelCopy panel{&s_mbar, 0};
-    if (!GLOBAL) panel.init();   // seen by the block behind the start vector's barriers
+    if (COPY) panel.init();   // seen by the block behind the start vector's barriers
     double *part0 = a.partials, *part1 = a.partials + 4 * (size_t)gridDim.x;
-    if (!GLOBAL && threadIdx.x < kBanks) xs[kSlicePW + threadIdx.x] = 0.0;
+    if (COPY && threadIdx.x < kBanks) xs[kSlicePW + threadIdx.x] = 0.0;
     // units of this block: an equal share of the cost; the direct forms keep
     // the units of a row (its chunks) in one block
     const uint64_t call = a.cpre[a.nu];
@@ -397,7 +412,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pi_slices(SliceArgs a) {
     const uint32_t U0 = block_unit(blockIdx.x), U1 = block_unit(blockIdx.x + 1);
     uint32_t wu0 = 0, wu1 = 0, R0 = 0, R1 = 0;
     if (!PANELS) {
-        warp_units(a, U0, U1, wid, wu0, wu1);
+        warp_units<kSliceWarps>(a, U0, U1, wid, wu0, wu1);
         if (U0 < U1) {
             R0 = a.unit[U0].y;
             R1 = U1 < a.nu ? a.unit[U1].y : n;
@@ -424,7 +439,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pi_slices(SliceArgs a) {
         }
         __syncthreads();
         double p[kSumK] = {s, 0, 0};
-        block_sum3_to(p, sm, part0 + 4 * (size_t)blockIdx.x);
+        block_sum3_to<kSliceWarps>(p, sm, part0 + 4 * (size_t)blockIdx.x);
         if (!bar.sync(&s_ok)) return;
         if (wid == 0) {
             grid_sum3(part0, s_sum);
@@ -446,8 +461,8 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pi_slices(SliceArgs a) {
             q += x * x;
         }
         double p2[kSumK] = {q, 0, 0};
-        if (!GLOBAL) asm volatile("fence.proxy.async;" ::: "memory");
-        block_sum3_to(p2, sm, part1 + 4 * (size_t)blockIdx.x);
+        if (COPY) asm volatile("fence.proxy.async;" ::: "memory");
+        block_sum3_to<kSliceWarps>(p2, sm, part1 + 4 * (size_t)blockIdx.x);
         if (!bar.sync(&s_ok)) return;
         if (wid == 0) grid_sum3(part1, s_sum);
         __syncthreads();
@@ -461,12 +476,12 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pi_slices(SliceArgs a) {
     double *src = a.va, *dst = a.vb;
     bool first = true;
     // this warp's first units: their stream starts before each barrier
-    Stream<GLOBAL, PANELS, WB> st;
+    Stream<FORM, WB> st;
     uint32_t p0 = 0, ue0 = 0;
     if (PANELS) {
         while (U0 < U1 && a.pan_u[p0 + 1] <= U0) p0++;
         ue0 = U0 < U1 && a.pan_u[p0 + 1] < U1 ? a.pan_u[p0 + 1] : U1;
-        warp_units(a, U0, ue0, wid, wu0, wu1);
+        warp_units<kSliceWarps>(a, U0, ue0, wid, wu0, wu1);
     }
     st.begin(a, wu0, wu1);
     // (direct) the first unit's row of this lane
@@ -482,7 +497,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pi_slices(SliceArgs a) {
     while (true) {
         // the iterate (its first panel); beside it one warp takes the last
         // iteration's sums
-        if (FORM == kFormShared) panel.issue(src, n, xs);
+        if (COPY && !PANELS) panel.issue(src, n < kSlicePW ? n : kSlicePW, xs);
         if (PANELS && U0 < U1)
             panel.issue(src + p0 * kSlicePW, n - p0 * kSlicePW < kSlicePW ? n - p0 * kSlicePW : kSlicePW, xs);
         if (!first && wid == kSliceWarps - 1) {
@@ -497,7 +512,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pi_slices(SliceArgs a) {
                 s_it[2] = s_sum[2] * inv;
             }
         }
-        if (FORM == kFormShared || (PANELS && U0 < U1))
+        if (COPY && (!PANELS || U0 < U1))
             if (!panel.wait() && lane == 0) atomicExch(a.err, 1u);
         __syncthreads();
         if (!first) {
@@ -517,7 +532,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pi_slices(SliceArgs a) {
                 }
                 double p[kSumK] = {uu, 0, 0};
                 __syncthreads();
-                block_sum3_to(p, sm, part + 4 * (size_t)blockIdx.x);
+                block_sum3_to<kSliceWarps>(p, sm, part + 4 * (size_t)blockIdx.x);
                 if (wid == 0) bar.arrive();
                 if (!bar.wait(&s_ok)) return;
                 if (blockIdx.x == 0 && wid == 0) {
@@ -553,7 +568,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pi_slices(SliceArgs a) {
             uint32_t p = p0, ue = ue0;
             while (true) {
                 double *y = a.y + (size_t)p * a.n32;
-                st.run(a, xs, [&](const uint4 &d, const uint4 &, double s) {
+                st.run(a, xs, src, [&](const uint4 &d, const uint4 &, bool, double s) {
                     const uint32_t lg = d.z >> 16;
                     if (d.w != 0xFFFFFFFFu) {
                         if (lane == 0) a.spart[d.w] = s;
@@ -567,7 +582,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pi_slices(SliceArgs a) {
                 while (a.pan_u[p + 1] <= u) p++;
                 ue = a.pan_u[p + 1] < U1 ? a.pan_u[p + 1] : U1;
                 uint32_t k0, k1;
-                warp_units(a, u, ue, wid, k0, k1);
+                warp_units<kSliceWarps>(a, u, ue, wid, k0, k1);
                 st.begin(a, k0, k1);
                 __syncthreads();   // every warp is done with the previous panel
                 panel.issue(src + p * kSlicePW, n - p * kSlicePW < kSlicePW ? n - p * kSlicePW : kSlicePW, xs);
@@ -576,17 +591,19 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pi_slices(SliceArgs a) {
             if (!bar.sync(&s_ok)) return;
             // the rows: their panels in order, then their chunks
             for (uint32_t i = gtid; i < n; i += gthr) {
+                const double xi = __ldcg(src + i), di = a.deg[i];
+                const uint32_t b = a.nslots ? a.sptr[i] : 0u, e = a.nslots ? a.sptr[i + 1] : 0u;
                 double acc = 0;
 #pragma unroll 4
                 for (uint32_t q = 0; q < a.P; q++) acc += __ldcg(a.y + (size_t)q * a.n32 + i);
-                if (a.nslots) {
-                    const uint32_t b = a.sptr[i], e = a.sptr[i + 1];
 #pragma unroll 4
-                    for (uint32_t q = b; q < e; q++) acc += __ldcg(a.spart + q);
-                }
-                fin(i, acc, __ldcg(src + i), a.deg[i]);
+                for (uint32_t q = b; q < e; q++) acc += __ldcg(a.spart + q);
+                fin(i, acc, xi, di);
             }
         } else {
+            auto own = [&](uint32_t i) -> double {
+                return FORM == kFormShared || (FORM == kFormHub && i < kSlicePW) ? xs[i] : src[i];
+            };
             // a row's own value and degree load one unit ahead of its sum
             uint32_t ri = 0;
             bool row = false;
@@ -597,19 +614,19 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pi_slices(SliceArgs a) {
                 row = d.w == 0xFFFFFFFFu && (lane & ((1u << lg) - 1u)) == 0 && ri < n;
                 if (row) {
                     di = __ldg(a.deg + ri);
-                    xi = GLOBAL ? src[ri] : xs[ri];
+                    xi = own(ri);
                 }
             };
             if (wu0 < wu1) {
                 ri = ri0;
                 row = row0;
                 di = di0;
-                if (row) xi = GLOBAL ? src[ri] : xs[ri];
+                if (row) xi = own(ri);
             }
-            st.run(a, GLOBAL ? src : xs, [&](const uint4 &d, const uint4 &dn, double s) {
+            st.run(a, xs, src, [&](const uint4 &d, const uint4 &dn, bool more, double s) {
                 if (row) fin(ri, s, xi, di);
                 else if (d.w != 0xFFFFFFFFu && lane == 0) a.spart[d.w] = s;
-                fetch(dn);
+                if (more) fetch(dn);
             });
             if (a.nslots) {
                 __syncthreads();   // the chunks of the block's rows are summed
@@ -618,13 +635,13 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pi_slices(SliceArgs a) {
                     if (b == e) continue;
                     double acc = 0;
                     for (uint32_t q = b; q < e; q++) acc += a.spart[q];
-                    fin(i, acc, GLOBAL ? src[i] : xs[i], a.deg[i]);
+                    fin(i, acc, own(i), a.deg[i]);
                 }
             }
         }
         // the iterate's next readers copy it through the async proxy
-        if (!GLOBAL) asm volatile("fence.proxy.async;" ::: "memory");
-        block_sum3_to(P, sm, part + 4 * (size_t)blockIdx.x);
+        if (COPY) asm volatile("fence.proxy.async;" ::: "memory");
+        block_sum3_to<kSliceWarps>(P, sm, part + 4 * (size_t)blockIdx.x);
         if (wid == 0) bar.arrive();
         st.begin(a, wu0, wu1);
         if (!bar.wait(&s_ok)) return;
@@ -683,6 +700,15 @@ __global__ void __launch_bounds__(256) k_sl_weights(uint32_t nitems, const uint3
         atomicAdd(stat, tot);
         atomicMax(stat + 1, mx);
     }
+}
+
+// entries of the leading kSlicePW rows in degree order
+__global__ void k_sl_lead(const uint32_t *rp, const uint32_t *inv, unsigned long long *out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned long long s = 0;
+    if (i < kSlicePW) s = rp[inv[i] + 1] - rp[inv[i]];
+    s = warp_sum(s);
+    if ((threadIdx.x & 31) == 0 && s) atomicAdd(out, s);
 }
 
 struct SliceBuild {
@@ -859,8 +885,10 @@ __global__ void __launch_bounds__(256) k_sl_groups(SliceBuild b) {
     }
 }
 
-// cost of a unit in the split over blocks and warps: its steps, plus the
-// price of two for the record, the butterfly and the row's value
+// cost of a unit in the split over blocks and warps, in half steps: its steps,
+// a quarter more where every lane has a row of its own (short rows share banks
+// more often: R-MAT 22's level 1 122 -> 118 us), plus the price of two steps for
+// the record, the butterfly and the row's value
 __global__ void __launch_bounds__(256) k_sl_units(SliceBuild b) {
     const unsigned lane = threadIdx.x & 31;
     const uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -888,7 +916,7 @@ __global__ void __launch_bounds__(256) k_sl_units(SliceBuild b) {
     if (!nu) return;
     if (r.chunks <= 1) {
         b.unit[u0] = make_uint4(off, i, r.steps | (r.lg << 16), 0xFFFFFFFFu);
-        b.ucost[u0] = r.steps + 2;
+        b.ucost[u0] = 2 * r.steps + (r.lg == 0 ? r.steps / 2 : 0) + 4;
         return;
     }
     uint32_t slot = b.sptr[i];
@@ -900,7 +928,7 @@ __global__ void __launch_bounds__(256) k_sl_units(SliceBuild b) {
     for (uint32_t k = 0; k < r.chunks; k++) {
         const uint32_t st = k + 1 < r.chunks ? full : r.steps - k * full;
         b.unit[u0 + k] = make_uint4(off + k * full, i, st | (5u << 16), slot + k);
-        b.ucost[u0 + k] = st + 2;
+        b.ucost[u0 + k] = 2 * st + 4;
     }
 }
 
@@ -1095,11 +1123,21 @@ __global__ void __launch_bounds__(32 * kLayWarps) k_sl_fill(SliceBuild b) {
 
 // ------------------------------------------------------------------ host --
 // levels of fewer mean entries per row and panel gather from L2 instead
-constexpr double kSliceMinSeg = 2.0;
+constexpr double kSliceMinSeg = 5.0;
 
-// The form of a level, before its rows are looked at.
-static SliceForm slice_form(uint32_t n, uint64_t m) {
+// levels whose gathers beyond the leading kSlicePW vertices in degree order
+// are at most this many take the hub form: panels cost a second barrier and a
+// pass over the rows' panel sums, about 5 us, a gather from L2 two clocks of an
+// SM
+constexpr uint64_t kHubTail = 1ull << 20;
+
+// The form of a level.  skew: its longest row is at least four times the mean;
+// tail: its entries beyond the leading kSlicePW vertices in degree order.
+// Mesh level of 57,210 vertices, 4.1 entries per row and panel: panels 12.6 us
+// an iteration, global 7.1; R-MAT 16's input level, 19 entries: 17 and 24.
+static SliceForm slice_form(uint32_t n, uint64_t m, bool skew, uint64_t tail) {
     if (n <= kSlicePW) return kFormShared;
+    if (skew && tail <= kHubTail) return kFormHub;
     const uint64_t P = cdiv(n, kSlicePW);
     if (P <= kSliceMaxPanels && (double)m >= kSliceMinSeg * (double)n * (double)P) return kFormPanels;
     return kFormGlobal;
@@ -1204,22 +1242,36 @@ int power_iter_slices(Context &C, const Level &L, const double *x_in, const uint
     // skewed levels are laid out in degree order: rows of a group then have
     // like lengths, and the most referenced columns share the first panels
     const double avg = (double)L.m / n;
-    SliceForm form = slice_form(n, L.m);
     const bool skew = maxlen >= 4.0 * avg && avg >= 4.0;
-    if (skew && form != kFormGlobal) {
+    uint64_t tail = 0;
+    if (skew) {
         uint32_t *perm, *inv;
         SGPB_TRY(degree_order(C, n, L.rp, &perm, &inv));
         b.perm = perm;
         b.inv = inv;
+        if (n > kSlicePW) {
+            unsigned long long *lead;
+            SGPB_TRY(dalloc_t(C, &lead, 1));
+            SGPB_TRY(dzero(C, lead, 8));
+            k_sl_lead<<<cdiv(kSlicePW, 256), 256, 0, C.stream>>>(L.rp, inv, lead);
+            C.kernel_launches++;
+            SGPB_TRY(read_u64(C, (const uint64_t *)lead, &tail));
+            tail = L.m - tail;
+        }
     }
+    const SliceForm form = slice_form(n, L.m, skew, tail);
+    if (form == kFormGlobal) b.perm = b.inv = nullptr;   // its gathers keep the level's locality
+    const bool wide = form == kFormGlobal || form == kFormHub;   // 32-bit destinations, places by rank
     b.direct = form != kFormPanels;
     b.P = form == kFormPanels ? cdiv(n, kSlicePW) : 1u;
     b.expand = form == kFormPanels && L.w && wtot <= 0xFFFFFFFFull && (double)wtot <= 1.25 * (double)L.m;
     const int wb = !L.w || b.expand ? 0 : wmax <= 0xFF ? 1 : wmax <= 0xFFFF ? 2 : wmax <= 0xFFFFFFFFull ? 4 : 8;
     const uint64_t me = b.expand ? wtot : L.m;
-    // entries per lane and unit: about two units a warp, 8 .. 64
+    // entries per lane and unit, 8 .. 64: units of at most a warp's share (with
+    // a quarter of it R-MAT 16's 6,915 vertices took 7.5 instead of 6.6 us an
+    // iteration, a mesh level of 190,000 14.3 instead of 10.5)
     uint32_t epl = 8;
-    while (epl < 64 && (uint64_t)epl * 2 * C.num_sms * kSliceWarps * 64 <= me) epl *= 2;
+    while (epl < 64 && (uint64_t)epl * 2 * C.num_sms * 16 * 16 <= me) epl *= 2;
     b.epl = epl;
     const size_t pn = (size_t)b.P * b.n32, pg = (size_t)b.P * b.ng;
     double *deg;
@@ -1238,7 +1290,7 @@ int power_iter_slices(Context &C, const Level &L, const double *x_in, const uint
     SGPB_TRY(dalloc_t(C, &b.rst, pn));
     const uint32_t lgrid = cdiv(b.nitems, kLayWarps) < (uint32_t)C.num_sms * 16 ? cdiv(b.nitems, kLayWarps)
                                                                               : (uint32_t)C.num_sms * 16;
-    const bool multi = form != kFormGlobal && maxlen > kSliceItem;
+    const bool multi = !wide && maxlen > kSliceItem;
     if (b.P > 1) {
         SGPB_TRY(dalloc_t(C, &b.tcol, L.m));
         SGPB_TRY(dzero(C, b.cnt, sizeof(uint32_t) * pn));
@@ -1279,13 +1331,13 @@ int power_iter_slices(Context &C, const Level &L, const double *x_in, const uint
     const uint32_t nu = h[2], nst = h[3], nslots = h[4];
     b.unb = unb; b.stb = stb; b.sptr = sptr;
     uint32_t *cpre;
-    const size_t cb = form == kFormGlobal ? 4 : 2;
+    const size_t cb = wide ? 4 : 2;
     SGPB_TRY(dalloc_t(C, &b.unit, (size_t)nu + 1));
     SGPB_TRY(dalloc_t(C, &b.ucost, (size_t)nu + 1));
     SGPB_TRY(dalloc_t(C, &cpre, (size_t)nu + 1));
     SGPB_TRY(dalloc_t(C, &b.pan_u, (size_t)b.P + 1));
     SGPB_TRY(dalloc(C, &b.ocol, (size_t)nst * 128 * cb));
-    if (form == kFormGlobal) SGPB_CUDA(cudaMemsetAsync(b.ocol, 0xFF, (size_t)nst * 128 * cb, C.stream));
+    if (wide) SGPB_CUDA(cudaMemsetAsync(b.ocol, 0xFF, (size_t)nst * 128 * cb, C.stream));
     if (wb) {
         SGPB_TRY(dalloc(C, &b.ow, (size_t)nst * 128 * wb));
         SGPB_TRY(dzero(C, b.ow, (size_t)nst * 128 * wb));
@@ -1293,13 +1345,13 @@ int power_iter_slices(Context &C, const Level &L, const double *x_in, const uint
     k_sl_units<<<cdiv(pg * 32, 256), 256, 0, C.stream>>>(b);
     C.kernel_launches++;
     SGPB_TRY(scan_u32(C, b.ucost, cpre, nu, nullptr));
-    if (form != kFormGlobal) {
+    if (!wide) {
         const uint32_t g = cdiv(nu, 8) < (uint32_t)C.num_sms * 16 ? cdiv(nu, 8) : (uint32_t)C.num_sms * 16;
         k_sl_preset<<<g, 256, 0, C.stream>>>(b, nu);
         C.kernel_launches++;
     }
-    if (L.wbytes == 8) SGPB_TRY(slice_fill<unsigned long long>(C, b, form == kFormGlobal, wb, lgrid));
-    else SGPB_TRY(slice_fill<uint32_t>(C, b, form == kFormGlobal, wb, lgrid));
+    if (L.wbytes == 8) SGPB_TRY(slice_fill<unsigned long long>(C, b, wide, wb, lgrid));
+    else SGPB_TRY(slice_fill<uint32_t>(C, b, wide, wb, lgrid));
     // the run
     a.n = n; a.n32 = b.n32; a.P = b.P; a.nu = nu; a.unit = b.unit; a.cpre = cpre; a.pan_u = b.pan_u;
     a.col = b.ocol; a.w = b.ow; a.sptr = sptr; a.nslots = nslots; a.deg = deg; a.inv = b.inv;
@@ -1324,13 +1376,15 @@ int power_iter_slices(Context &C, const Level &L, const double *x_in, const uint
     a.iter_max = iter_max;
     a.iter0 = iter0;
     a.dot0 = dot0;
-    uint32_t grid = cdiv(nu, kSliceWarps);
+    const int threads = slice_threads(form, wb);
+    uint32_t grid = cdiv(nu, (uint32_t)threads / 32);
     if (grid > (uint32_t)C.num_sms) grid = C.num_sms;
     if (C.grid_cap && grid > C.grid_cap) grid = C.grid_cap;
     if (grid < 1) grid = 1;
     SGPB_TRY(dalloc_t(C, &a.partials, (size_t)8 * grid));
     const void *k = form == kFormShared   ? slice_kernel<kFormShared>(wb)
                     : form == kFormGlobal ? slice_kernel<kFormGlobal>(wb)
+                    : form == kFormHub    ? slice_kernel<kFormHub>(wb)
                                           : slice_kernel<kFormPanels>(wb);
     const size_t dyn = form == kFormGlobal ? 0 : kSliceSmem;
     if (dyn) SGPB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSliceSmem));
@@ -1342,7 +1396,7 @@ int power_iter_slices(Context &C, const Level &L, const double *x_in, const uint
     } evfree{ev};
     SGPB_CUDA(cudaEventRecord(ev[0], C.stream));
     void *args[] = {&a};
-    SGPB_CUDA(cudaLaunchCooperativeKernel(k, dim3(grid), dim3(kSliceThreads), args, dyn, C.stream));
+    SGPB_CUDA(cudaLaunchCooperativeKernel(k, dim3(grid), dim3((unsigned)threads), args, dyn, C.stream));
     C.kernel_launches++;
     SGPB_CUDA(cudaEventRecord(ev[1], C.stream));
     SGPB_CUDA(cudaMemcpyAsync(C.h_pinned, res_d, 6 * sizeof(double), cudaMemcpyDeviceToHost, C.stream));

@@ -1,7 +1,7 @@
 """Power iteration on row slices (slices.cu) at the edges of its forms: the
-iterate in one block's shared memory (up to 25,600 vertices), column panels
-(wider levels of at least two entries per row and panel) and the global
-gather; rows of every lane split, rows of several chunks and of several layout
+iterate in one block's shared memory (up to 25,600 vertices), its leading part
+there (skewed levels of few entries beyond it), column panels (wider levels of
+at least five entries per row and panel) and the global gather; rows of every lane split, rows of several chunks and of several layout
 items, unit, repeated, 8-, 16-, 32- and 64-bit weights, rows without entries.
 Against the oracle after a fixed number of iterations: each iteration rounds
 the FP64 iterate to about 1e-16 per operation, so 40 of them stay well within
@@ -69,17 +69,18 @@ def skewed(n, m, seed):
     return csr(n, np.concatenate([u, np.zeros(hub.size, np.int64)]), np.concatenate([v, hub]))
 
 
-@pytest.mark.parametrize("n,m", [(4001, 30000), (25600, 400000), (25601, 400000), (51203, 1500000), (77000, 200000)])
+@pytest.mark.parametrize("n,m", [(4001, 30000), (25600, 400000), (25601, 400000), (51203, 1500000), (77000, 200000),
+                                 (51201, 6000000)])
 @pytest.mark.parametrize("top", [0, 200, 60000, 1 << 31])
 def test_forms_and_weights(partitioner, n, m, top):
-    """One panel exactly full, one vertex more, three panels, and a sparse
-    level (global gather), unit weights and every weight width."""
+    """One panel exactly full, one vertex more, three panels' width of few and
+    of many entries, and a sparse level, unit weights and every weight width."""
     rp, col = skewed(n, m, n)
     check(partitioner, rp, col, weights(rp, col, top) if top else None)
 
 
 def test_wide_weights(partitioner):
-    for n, m in ((9000, 120000), (60000, 900000)):
+    for n, m in ((9000, 120000), (60000, 900000), (51201, 6000000)):
         rp, col = skewed(n, m, 3)
         check(partitioner, rp, col, weights(rp, col, (1 << 33) + 5), wide=True)
 
@@ -87,10 +88,8 @@ def test_wide_weights(partitioner):
 def test_repeated_weights(partitioner):
     """Panels of a level whose total weight is within 1.25 of its entries:
     entries are repeated (several copies of one destination in a row)."""
-    rp, col = skewed(70001, 2000000, 5)
-    w = weights(rp, col, 9)
-    w[w < 9] = 1
-    w[w == 9] = np.where(np.isin(col[w == 9] % 2, (0,)), 1, 1)
+    rp, col = skewed(70001, 8000000, 5)
+    w = np.ones(col.size, np.uint64)
     rows = np.repeat(np.arange(70001), np.diff(rp).astype(np.int64))
     w[(rows % 64 == 0) & (col % 64 == 0)] = 37
     assert w.sum() <= 1.25 * w.size and w.max() == 37
