@@ -2666,10 +2666,14 @@ int power_iter_level(Context &C, const Level &Lin, const double *x_in, const uin
     // needs no layout, and goes on from their iterate only if it has to.
     const bool slices = power_iter_slices_ok(Lin, o);
     const bool probe = slices && o.probe && Lin.m >= kProbeMinM;
+    // A layout that does not fit the device leaves the level to that kernel.
+    bool fits = true;
     if (slices && !probe) {
-        SGPB_TRY(power_iter_slices(C, Lin, x_in, vcmap, x_out, o, iter_budget(n, o), 0, 0.0, res));
-        if (want_residual) SGPB_TRY(level_residual(C, Lin, x_out, o.normlap, res));
-        return SGP_B200_OK;
+        SGPB_TRY(power_iter_slices(C, Lin, x_in, vcmap, x_out, o, iter_budget(n, o), 0, 0.0, res, &fits));
+        if (fits) {
+            if (want_residual) SGPB_TRY(level_residual(C, Lin, x_out, o.normlap, res));
+            return SGP_B200_OK;
+        }
     }
     PIArgs a;
     memset(&a, 0, sizeof(a));
@@ -2751,10 +2755,15 @@ int power_iter_level(Context &C, const Level &Lin, const double *x_in, const uin
     if (a.iter_max < imax && rh[4] != 0.0) {
         // not converged: repeat the last iteration from the vector it began
         // with, the dot product before it carried over
-        SGPB_TRY(power_iter_slices(C, Lin, x_out, nullptr, x_out, o, imax, kProbeIters - 1, rh[6], res));
-        res->kernel_ms += kms;
-        if (want_residual) SGPB_TRY(level_residual(C, Lin, x_out, o.normlap, res));
-        return SGP_B200_OK;
+        SGPB_TRY(power_iter_slices(C, Lin, x_out, nullptr, x_out, o, imax, kProbeIters - 1, rh[6], res, &fits));
+        if (fits) {
+            res->kernel_ms += kms;
+            if (want_residual) SGPB_TRY(level_residual(C, Lin, x_out, o.normlap, res));
+            return SGP_B200_OK;
+        }
+        a.iter_max = imax;
+        SGPB_TRY(run_pi(C, L, a, mixed, want_panels ? &panels : nullptr, res_d, rh, &kms,
+                        pi_grid(C, n, L.m, tune.units), tune.mode));
     }
     const uint64_t total_iters = (uint64_t)rh[0];
     res->niter = total_iters;

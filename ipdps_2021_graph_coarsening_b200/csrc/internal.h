@@ -58,6 +58,7 @@ struct Context {
     float t_map = 0, t_build = 0;   // coarsening of the last partition: HEC mapping / coarse builds
     uint32_t kernel_launches = 0;
     std::string dev_key;            // device name, SM count and compute capability (autotuner cache key)
+    bool out_of_memory = false;     // an allocation failed for want of memory
     uint32_t grid_cap = 0;          // > 0: at most this many blocks per power-iteration launch
 };
 
@@ -183,10 +184,12 @@ int power_iter_level(Context &C, const Level &L, const double *x_in, const uint3
 // The same recurrence on row slices (slices.cu): FP64 levels of any size.
 // iter0 / dot0: iterations already done on the vector x_in and the dot
 // product before its last one (0 and 0 for a fresh start); their number counts
-// towards iter_max and the result's niter.
+// towards iter_max and the result's niter.  *fits = false: the layout did not
+// fit the device, nothing was done.
 bool power_iter_slices_ok(const Level &L, const PowerIterOpts &o);
 int power_iter_slices(Context &C, const Level &L, const double *x_in, const uint32_t *vcmap, double *x_out,
-                      const PowerIterOpts &o, uint64_t iter_max, uint64_t iter0, double dot0, PowerIterResult *res);
+                      const PowerIterOpts &o, uint64_t iter_max, uint64_t iter0, double dot0, PowerIterResult *res,
+                      bool *fits);
 // order of the vertices by descending degree class (eight classes an octave),
 // stable inside a class: perm (vertex -> new id) and inv
 int degree_order(Context &C, uint32_t n, const uint32_t *rp, uint32_t **perm, uint32_t **inv);

@@ -1125,6 +1125,10 @@ __global__ void __launch_bounds__(32 * kLayWarps) k_sl_fill(SliceBuild b) {
 // levels of fewer mean entries per row and panel gather from L2 instead
 constexpr double kSliceMinSeg = 5.0;
 
+// largest weight that is laid out as copies of its entry (R-MAT 22's level 1
+// has 160)
+constexpr uint64_t kMaxCopies = 4096;
+
 // levels whose gathers beyond the leading kSlicePW vertices in degree order
 // are at most this many take the hub form: panels cost a second barrier and a
 // pass over the rows' panel sums, about 5 us, a gather from L2 two clocks of an
@@ -1184,10 +1188,11 @@ static int slice_fill(Context &C, const SliceBuild &b, bool wide, int wb, uint32
     return SGP_B200_OK;
 }
 
-int power_iter_slices(Context &C, const Level &L, const double *x_in, const uint32_t *vcmap, double *x_out,
-                      const PowerIterOpts &o, uint64_t iter_max, uint64_t iter0, double dot0, PowerIterResult *res) {
+// Lays the level out and runs it; *tight: the layout did not fit, nothing ran.
+static int slices_run(Context &C, const Level &L, const double *x_in, const uint32_t *vcmap, double *x_out,
+                      const PowerIterOpts &o, uint64_t iter_max, uint64_t iter0, double dot0, PowerIterResult *res,
+                      bool *tight) {
     const uint32_t n = L.n;
-    const size_t mark = C.owned.size();
     SliceBuild b;
     memset(&b, 0, sizeof(b));
     SliceArgs a;
@@ -1264,7 +1269,9 @@ int power_iter_slices(Context &C, const Level &L, const double *x_in, const uint
     const bool wide = form == kFormGlobal || form == kFormHub;   // 32-bit destinations, places by rank
     b.direct = form != kFormPanels;
     b.P = form == kFormPanels ? cdiv(n, kSlicePW) : 1u;
-    b.expand = form == kFormPanels && L.w && wtot <= 0xFFFFFFFFull && (double)wtot <= 1.25 * (double)L.m;
+    // (one lane writes an entry's copies: at most kMaxCopies)
+    b.expand = form == kFormPanels && L.w && wmax <= kMaxCopies && wtot <= 0xFFFFFFFFull &&
+               (double)wtot <= 1.25 * (double)L.m;
     const int wb = !L.w || b.expand ? 0 : wmax <= 0xFF ? 1 : wmax <= 0xFFFF ? 2 : wmax <= 0xFFFFFFFFull ? 4 : 8;
     const uint64_t me = b.expand ? wtot : L.m;
     // entries per lane and unit, 8 .. 64: units of at most a warp's share (with
@@ -1332,6 +1339,11 @@ int power_iter_slices(Context &C, const Level &L, const double *x_in, const uint
     b.unb = unb; b.stb = stb; b.sptr = sptr;
     uint32_t *cpre;
     const size_t cb = wide ? 4 : 2;
+    if (const char *e = getenv("SGPB_PI_SLICES_MB"))   // a limit on the laid-out matrix
+        if (*e && (uint64_t)nst * 128 * (cb + wb) > strtoull(e, nullptr, 10) << 20) {
+            *tight = true;
+            return SGP_B200_ERR_DEVICE;
+        }
     SGPB_TRY(dalloc_t(C, &b.unit, (size_t)nu + 1));
     SGPB_TRY(dalloc_t(C, &b.ucost, (size_t)nu + 1));
     SGPB_TRY(dalloc_t(C, &cpre, (size_t)nu + 1));
@@ -1416,10 +1428,21 @@ int power_iter_slices(Context &C, const Level &L, const double *x_in, const uint
     float t = 0;
     cudaEventElapsedTime(&t, ev[0], ev[1]);
     res->kernel_ms = t;
+    return SGP_B200_OK;
+}
+
+int power_iter_slices(Context &C, const Level &L, const double *x_in, const uint32_t *vcmap, double *x_out,
+                      const PowerIterOpts &o, uint64_t iter_max, uint64_t iter0, double dot0, PowerIterResult *res,
+                      bool *fits) {
+    const size_t mark = C.owned.size();
+    bool tight = false;
+    C.out_of_memory = false;
+    const int rc = slices_run(C, L, x_in, vcmap, x_out, o, iter_max, iter0, dot0, res, &tight);
     // the layout is this call's alone: give it back before the next level
     for (size_t q = mark; q < C.owned.size(); q++) cudaFreeAsync(C.owned[q], C.stream);
     C.owned.resize(mark);
-    return SGP_B200_OK;
+    *fits = rc == SGP_B200_OK || !(tight || C.out_of_memory);
+    return *fits ? rc : SGP_B200_OK;
 }
 
 }  // namespace sgpb

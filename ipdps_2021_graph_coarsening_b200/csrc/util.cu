@@ -30,6 +30,10 @@ int dalloc(Context &C, void **p, size_t bytes) {
     cudaError_t e = cudaMallocAsync(p, bytes, C.stream);
     if (e != cudaSuccess) {
         set_error("device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+        if (e == cudaErrorMemoryAllocation) {
+            C.out_of_memory = true;
+            cudaGetLastError();   // the caller may go on without the buffer
+        }
         return SGP_B200_ERR_DEVICE;
     }
     C.owned.push_back(*p);

@@ -96,6 +96,37 @@ def test_repeated_weights(partitioner):
     check(partitioner, rp, col, w)
 
 
+def test_one_heavy_entry(partitioner):
+    """The same with one weight far above the others: not repeated."""
+    rp, col = skewed(70001, 8000000, 5)
+    rows = np.repeat(np.arange(70001), np.diff(rp).astype(np.int64))
+    e = int(np.flatnonzero(rows < col)[1000])
+    w = np.ones(col.size, np.uint64)
+    w[((rows == rows[e]) & (col == col[e])) | ((rows == col[e]) & (col == rows[e]))] = 4097
+    assert w.sum() <= 1.25 * w.size and w.max() == 4097
+    check(partitioner, rp, col, w)
+
+
+@pytest.mark.parametrize("name", ["coarse", "finest"])
+def test_layout_does_not_fit(partitioner, monkeypatch, name):
+    """A level whose layout is refused runs on the main kernel: from its start
+    vector, and after a finest level's first iterations."""
+    monkeypatch.setenv("SGPB_PI_SLICES_MB", "0")
+    if name == "coarse":
+        rp, col = skewed(30001, 400000, 2)
+        check(partitioner, rp, col, weights(rp, col, 200))
+        return
+    g = G.erdos_renyi(150001, 8.0, seed=9)
+    a = partitioner.partition(g, rng_state=5)
+    monkeypatch.delenv("SGPB_PI_SLICES_MB")
+    monkeypatch.setenv("SGPB_PI_SLICES", "0")
+    b = partitioner.partition(g, rng_state=5)
+    assert a.level_n == b.level_n and a.level_iters[0] > 4
+    assert all(abs(x - y) <= 2 for x, y in zip(a.level_iters, b.level_iters))
+    assert abs(a.lam - b.lam) <= 1e-9 * abs(b.lam)
+    assert abs(a.edgecut - b.edgecut) <= 0.001 * b.edgecut
+
+
 @pytest.mark.parametrize("n", [9001, 60001])
 def test_long_rows(partitioner, n):
     """Two hubs joined to every vertex: rows of several chunks and of several
