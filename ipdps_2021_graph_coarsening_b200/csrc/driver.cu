@@ -82,13 +82,12 @@ static int stage_input(Context &C, const sgp_b200_graph_t *g, Level *L0) {
     } else {
         SGPB_TRY(dalloc_t(C, &L0->rp, (size_t)g->n + 1));
         SGPB_TRY(dalloc_t(C, &L0->col, (size_t)g->m + 1));
-        SGPB_CUDA(cudaMemcpyAsync(L0->rp, g->row_ptr, sizeof(uint32_t) * ((size_t)g->n + 1), cudaMemcpyHostToDevice,
-                                  C.stream));
-        SGPB_CUDA(cudaMemcpyAsync(L0->col, g->col, sizeof(uint32_t) * g->m, cudaMemcpyHostToDevice, C.stream));
+        SGPB_TRY(upload_host(C, L0->rp, g->row_ptr, sizeof(uint32_t) * ((size_t)g->n + 1)));
+        SGPB_TRY(upload_host(C, L0->col, g->col, sizeof(uint32_t) * g->m));
         if (g->w) {
             uint32_t *w;
             SGPB_TRY(dalloc_t(C, &w, (size_t)g->m + 1));
-            SGPB_CUDA(cudaMemcpyAsync(w, g->w, sizeof(uint32_t) * g->m, cudaMemcpyHostToDevice, C.stream));
+            SGPB_TRY(upload_host(C, w, g->w, sizeof(uint32_t) * g->m));
             L0->w = w;
         }
     }

@@ -48,7 +48,7 @@ struct Context {
     int num_sms = 0;
     size_t smem_optin = 0;
     uint64_t *h_pinned = nullptr;   // small pinned staging area for scalar read-backs
-    uint8_t *h_stage = nullptr;     // pinned ring for streaming host bytes to the device (mtx.cu)
+    uint8_t *h_stage = nullptr;     // pinned ring for streaming host bytes to and from the device (mtx.cu)
     size_t h_stage_slot = 0;        // bytes per ring slot
     cudaEvent_t stage_ev[4] = {};   // copy of each slot done
     std::vector<void *> owned;      // allocations released at the end of a call
@@ -69,6 +69,9 @@ template <typename T>
 int dalloc_t(Context &C, T **p, size_t count) { return dalloc(C, (void **)p, count * sizeof(T)); }
 int dzero(Context &C, void *p, size_t bytes);
 void release_all(Context &C);
+// host bytes to the device on the context's stream; src is read when this
+// returns if it is pageable, when the stream is done if it is pinned (mtx.cu)
+int upload_host(Context &C, void *dst, const void *src, size_t bytes);
 
 // device-wide exclusive scan of n uint32 counts into uint32 offsets[n+1]
 // (out[n] = total).  Returns SGP_B200_ERR_TOO_LARGE when the total does not

@@ -79,7 +79,12 @@ constexpr uint32_t kNoEdge = 0xFFFFFFFFu;
 constexpr unsigned long long kNoKey = ~0ull;   // sorts after every entry key
 constexpr int kMaxBanners = 16;
 constexpr int kStageSlots = 4;
-constexpr size_t kStageSlotBytes = (size_t)32 << 20;
+constexpr size_t kStageSlotBytes = (size_t)32 << 20;   // largest slot
+
+// pageable arrays from this size on are uploaded through the ring, in slots of
+// at most kUploadSlotBytes (a context's first one pays for the ring, about
+// 0.3 ms a MiB of slot)
+constexpr size_t kUploadMin = (size_t)16 << 20, kUploadSlotBytes = (size_t)8 << 20;
 
 enum : uint32_t { kLineSyntax = 1, kLineZero = 2, kLineRange = 3 };
 
@@ -574,10 +579,10 @@ class HostPool {
     uint64_t gen_ = 0;
 };
 
-// dst[0, n) = src[0, n) in pool-sized pieces of at least 1 MiB
+// dst[0, n) = src[0, n) in pool-sized pieces of at least 512 KiB
 static void par_copy(void *dst, const void *src, size_t n) {
     HostPool &P = HostPool::get();
-    const size_t min_piece = (size_t)1 << 20;
+    const size_t min_piece = (size_t)1 << 19;
     int parts = (int)((n + min_piece - 1) / min_piece);
     if (parts > P.width()) parts = P.width();
     if (parts <= 1) {
@@ -615,11 +620,30 @@ static bool par_pread(int fd, uint8_t *buf, size_t n, uint64_t off) {
     return ok.load();
 }
 
-static int ensure_stage(Context &C) {
-    if (C.h_stage) return SGP_B200_OK;
-    SGPB_CUDA(cudaMallocHost((void **)&C.h_stage, kStageSlots * kStageSlotBytes));
-    C.h_stage_slot = kStageSlotBytes;
-    for (int i = 0; i < kStageSlots; i++) SGPB_CUDA(cudaEventCreateWithFlags(&C.stage_ev[i], cudaEventDisableTiming));
+// Bytes per ring slot for a transfer of `len` bytes: a power of two from 1 MiB
+// to `top`, about an eighth of the transfer, so that filling one slot overlaps
+// the copies of others (32 MB slots held a 13 MB text whole: the converter's
+// call 5.5 -> 5.2 ms, a context's first one, which pins the ring, 57 -> 9).
+static size_t stage_slot(uint64_t len, size_t top) {
+    size_t c = (size_t)1 << 20;
+    while (c < top && c * 8 < len) c *= 2;
+    return c;
+}
+
+// the pinned ring, with slots of at least `slot` bytes
+static int ensure_stage(Context &C, size_t slot) {
+    if (C.h_stage && C.h_stage_slot >= slot) return SGP_B200_OK;
+    if (C.h_stage) {
+        SGPB_CUDA(cudaStreamSynchronize(C.stream));
+        cudaFreeHost(C.h_stage);
+        C.h_stage = nullptr;
+    }
+    uint8_t *ring = nullptr;
+    SGPB_CUDA(cudaMallocHost((void **)&ring, kStageSlots * slot));
+    C.h_stage = ring;
+    C.h_stage_slot = slot;
+    for (int i = 0; i < kStageSlots; i++)
+        if (!C.stage_ev[i]) SGPB_CUDA(cudaEventCreateWithFlags(&C.stage_ev[i], cudaEventDisableTiming));
     return SGP_B200_OK;
 }
 
@@ -628,6 +652,13 @@ static bool is_pinned(const void *p) {
     const bool pinned = cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeHost;
     cudaGetLastError();
     return pinned;
+}
+
+static bool is_pageable(const void *p) {
+    cudaPointerAttributes at;
+    const bool plain = cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    return plain;
 }
 
 // The whole text into `dtext` (capacity >= len): pinned host memory and device
@@ -642,10 +673,11 @@ static int upload_text(Context &C, MtxSource &src, uint8_t *dtext) {
         SGPB_CUDA(cudaMemcpyAsync(dtext, src.host, src.len, cudaMemcpyHostToDevice, C.stream));
         return SGP_B200_OK;
     }
-    SGPB_TRY(ensure_stage(C));
+    const size_t chunk = stage_slot(src.len, kStageSlotBytes);
+    SGPB_TRY(ensure_stage(C, chunk));
     int slot = 0;
-    for (uint64_t off = 0; off < src.len; off += C.h_stage_slot, slot = (slot + 1) % kStageSlots) {
-        const size_t n = (size_t)(src.len - off < C.h_stage_slot ? src.len - off : C.h_stage_slot);
+    for (uint64_t off = 0; off < src.len; off += chunk, slot = (slot + 1) % kStageSlots) {
+        const size_t n = (size_t)(src.len - off < chunk ? src.len - off : chunk);
         uint8_t *buf = C.h_stage + (size_t)slot * C.h_stage_slot;
         SGPB_CUDA(cudaEventSynchronize(C.stage_ev[slot]));
         if (src.f) {
@@ -662,6 +694,33 @@ static int upload_text(Context &C, MtxSource &src, uint8_t *dtext) {
     return SGP_B200_OK;
 }
 
+// A host array to the device: pinned and small arrays in one copy, large
+// pageable ones through the pinned ring.  The runtime stages pageable memory
+// on one thread, about 11 GB/s: the coarsening call on R-MAT 20 (122 MB of
+// destinations) 16.3 -> 7.9 ms, of R-MAT 19 9.2 -> 5.4, R-MAT 18 4.7 -> 4.0.
+int upload_host(Context &C, void *dst, const void *src, size_t bytes) {
+    const size_t chunk = stage_slot(bytes, kUploadSlotBytes);
+    if (bytes < kUploadMin || !is_pageable(src) || ensure_stage(C, chunk) != SGP_B200_OK) {
+        cudaGetLastError();   // no pinned ring to be had
+        SGPB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, C.stream));
+        return SGP_B200_OK;
+    }
+    int slot = 0;
+    for (size_t off = 0; off < bytes; off += chunk, slot = (slot + 1) % kStageSlots) {
+        const size_t n = bytes - off < chunk ? bytes - off : chunk;
+        uint8_t *buf = C.h_stage + (size_t)slot * C.h_stage_slot;
+        SGPB_CUDA(cudaEventSynchronize(C.stage_ev[slot]));
+        try {
+            par_copy(buf, (const char *)src + off, n);
+        } catch (...) {   // no threads to be had
+            memcpy(buf, (const char *)src + off, n);
+        }
+        SGPB_CUDA(cudaMemcpyAsync((char *)dst + off, buf, n, cudaMemcpyHostToDevice, C.stream));
+        SGPB_CUDA(cudaEventRecord(C.stage_ev[slot], C.stream));
+    }
+    return SGP_B200_OK;
+}
+
 // Device -> pageable host through the pinned ring: the copy of one slot out
 // (by the host pool) overlaps the transfers into the others.
 struct CopySeg {
@@ -670,7 +729,10 @@ struct CopySeg {
     size_t bytes;
 };
 static int download_staged(Context &C, const CopySeg *segs, int nseg) {
-    SGPB_TRY(ensure_stage(C));
+    uint64_t len = 0;
+    for (int i = 0; i < nseg; i++) len += segs[i].bytes;
+    const size_t chunk = stage_slot(len, kStageSlotBytes);
+    SGPB_TRY(ensure_stage(C, chunk));
     struct Chunk {
         char *dst;
         const char *src;
@@ -678,9 +740,9 @@ static int download_staged(Context &C, const CopySeg *segs, int nseg) {
     };
     std::vector<Chunk> ch;
     for (int i = 0; i < nseg; i++)
-        for (size_t o = 0; o < segs[i].bytes; o += C.h_stage_slot)
+        for (size_t o = 0; o < segs[i].bytes; o += chunk)
             ch.push_back({(char *)segs[i].dst + o, (const char *)segs[i].src + o,
-                          segs[i].bytes - o < C.h_stage_slot ? segs[i].bytes - o : C.h_stage_slot});
+                          segs[i].bytes - o < chunk ? segs[i].bytes - o : chunk});
     const int K = (int)ch.size();
     auto issue = [&](int k) -> int {
         const int slot = k % kStageSlots;
