@@ -1787,10 +1787,19 @@ struct MidLevelDesc {
     const uint32_t *vcmap;
     double *out;             // normalised result (n)
     double *va, *vb, *deg;   // iterate buffers and weighted degrees (n each)
+    uint4 *rows;             // [mid_tiles(m, blocks)][32] rows of each lane's entries (mid_plan)
     double tol;
     uint64_t iter_max;
     double *res;             // [0] niter [1] dot [2] gb [3] lambda [4] capped [6] ms
 };
+
+// Tiles of kTile entries from the multiple of four at or below a warp's first
+// one: the first tile of the g-th warp of a level, and room for all of them.  A
+// warp of the entries [a, b) has at most (b - a + 130) / kTile of them.
+__host__ __device__ __forceinline__ uint64_t mid_tile0(uint64_t first_entry, uint32_t g) {
+    return first_entry / kTile + 3ull * g;
+}
+static uint64_t mid_tiles(uint64_t m, uint32_t blocks) { return mid_tile0(m, blocks * kMidWarps) + 3; }
 
 // first row i in [lo, hi] with rp[i] >= t
 __device__ __forceinline__ uint32_t rows_at(const uint32_t *rp, uint32_t lo, uint32_t hi, uint64_t t) {
@@ -1829,9 +1838,176 @@ __device__ __forceinline__ void cluster_sum(double (&v)[NV], double (*slot)[8], 
     __syncthreads();   // sm is reused by the next sum
 }
 
+// The rows of the entries of a warp's tiles, once per level: lane l of a tile
+// holds entries c + 4 l .. c + 4 l + 3.  Bit 31 of lane 31's last row: its row
+// goes on in the next tile (a level has fewer than 2^31 rows).
+__device__ __forceinline__ void mid_plan(const uint32_t *rp, uint32_t ra, uint32_t rb, uint4 *rows) {
+    const unsigned lane = threadIdx.x & 31;
+    if (ra >= rb) return;
+    const uint32_t Ea = rp[ra], Eb = rp[rb];
+    for (uint64_t c = Ea & ~3u; c < Eb; c += kTile, rows += 32) {
+        uint32_t r[4] = {0, 0, 0, 0};
+        uint32_t s = 0;
+        bool have = false;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint64_t q = c + 4 * lane + k;
+            if (q < Ea || q >= Eb) continue;
+            if (!have) {
+                uint32_t lo = ra, hi = rb - 1;   // last row that begins at or before q
+                while (lo < hi) {
+                    const uint32_t mid = lo + ((hi - lo + 1) >> 1);
+                    if (rp[mid] <= q) lo = mid;
+                    else hi = mid - 1;
+                }
+                s = lo;
+                have = true;
+            } else {
+                while (rp[s + 1] <= q) s++;
+            }
+            r[k] = s;
+        }
+        if (lane == 31 && have && rp[s + 1] > c + kTile) r[3] |= 0x80000000u;
+        rows[lane] = make_uint4(r[0], r[1], r[2], r[3]);
+    }
+}
+
+// Streams a warp's planned tiles: fin(i, sum, degree, own value) is called once
+// per row with entries.  A row's terms are added in the order of warp_stream
+// (four entries a lane, a segmented scan over the lanes, a carry between
+// tiles).  Two tiles are in flight: destinations, weights and rows are loaded
+// two ahead, the iterate's and the rows' own values and degrees one ahead, so a
+// tile waits for neither L2 nor the row search (XXX).
+template <bool MX, typename W, typename ACC, typename Fin>
+__device__ __forceinline__ void mid_stream(const uint32_t *rp, const uint32_t *col, const W *w, const double *src,
+                                           const double *deg, uint64_t m, bool vec, uint32_t ra, uint32_t rb,
+                                           const uint4 *rows, Fin &fin) {
+    const unsigned lane = threadIdx.x & 31;
+    if (ra >= rb) return;
+    const uint32_t Ea = rp[ra], Eb = rp[rb];
+    if (Ea == Eb) return;
+    const uint32_t c0 = Ea & ~3u;
+    const uint32_t tiles = (uint32_t)(((uint64_t)Eb - c0 + kTile - 1) / kTile);
+    struct Tile {
+        uint32_t cc[4];
+        W ww[4];
+        uint4 r;
+    };
+    struct Vals {
+        double xg[4], xs[4], dg[4];
+    };
+    auto in = [&](uint32_t t, int k) -> bool {
+        const uint32_t q = t * kTile + 4 * lane + k;   // from c0; a row has fewer than 2^31 entries
+        return q >= Ea - c0 && q < Eb - c0;
+    };
+    auto row_of = [](const uint4 &r, int k) -> uint32_t {
+        return k == 0 ? r.x : k == 1 ? r.y : k == 2 ? r.z : r.w & 0x7FFFFFFFu;
+    };
+    auto load = [&](uint32_t t, Tile &T) {
+        load4<true, W>(col, w, c0 + t * kTile + 4 * lane, m, vec, T.cc, T.ww);
+        T.r = rows[(size_t)t * 32 + lane];
+    };
+    auto gather = [&](uint32_t t, const Tile &T, Vals &V) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const bool ok = in(t, k);
+            const uint32_t i = row_of(T.r, k);
+            V.xg[k] = ok ? src[T.cc[k]] : 0.0;
+            V.xs[k] = ok ? src[i] : 0.0;
+            V.dg[k] = ok ? deg[i] : 0.0;
+        }
+    };
+    Tile cur, nxt;
+    Vals v;
+    load(0, cur);
+    nxt = cur;
+    if (tiles > 1) load(1, nxt);
+    gather(0, cur, v);
+    ACC carry = 0;
+    for (uint32_t t = 0; t < tiles; t++) {
+        Vals vn = v;
+        Tile nn = nxt;
+        if (t + 1 < tiles) gather(t + 1, nxt, vn);
+        if (t + 2 < tiles) load(t + 2, nn);
+        // the entries' terms (mixed: edge differences to the row's own value)
+        ACC prod[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if constexpr (MX) prod[k] = in(t, k) ? spmv_term<true, ACC>(w != nullptr, v.xs[k], v.xg[k], w ? cur.ww[k] : (W)0) : (ACC)0;
+            else prod[k] = (ACC)(w ? (double)cur.ww[k] * v.xg[k] : v.xg[k]);
+        }
+        const unsigned lane_first = t == 0 ? (Ea - c0) >> 2 : 0u;
+        ACC A = 0, B = 0, run = 0;
+        uint32_t r0 = 0, rs = 0;
+        double x0 = 0, d0 = 0, xr = 0, dr = 0;
+        bool started = false, multi = false;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (!in(t, k)) continue;
+            const uint32_t i = row_of(cur.r, k);
+            if (!started) {
+                started = true;
+                r0 = rs = i;
+                x0 = xr = v.xs[k];
+                d0 = dr = v.dg[k];
+                run = prod[k];
+            } else if (i != rs) {
+                if (!multi) {
+                    A = run;
+                    multi = true;
+                } else {
+                    fin(rs, run, dr, xr);   // middle run
+                }
+                rs = i;
+                xr = v.xs[k];
+                dr = v.dg[k];
+                run = prod[k];
+            } else {
+                run += prod[k];
+            }
+        }
+        B = run;
+        if (!multi) A = B;
+        if (lane == lane_first && started) {
+            A += carry;
+            if (!multi) B = A;
+        }
+        // segmented inclusive scan over lanes of the last-run sums
+        const uint32_t prev_rs = __shfl_up_sync(0xFFFFFFFFu, rs, 1);
+        const int prev_v = __shfl_up_sync(0xFFFFFFFFu, (int)started, 1);
+        const bool cont_prev = started && lane > 0 && prev_v && lane != lane_first && prev_rs == r0;
+        ACC Sc = started ? B : (ACC)0;
+        int F = (!started || multi || !cont_prev) ? 1 : 0;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const ACC x = __shfl_up_sync(0xFFFFFFFFu, Sc, d);
+            const int xf = __shfl_up_sync(0xFFFFFFFFu, F, d);
+            if (lane >= (unsigned)d) {
+                if (!F) Sc += x;
+                F |= xf;
+            }
+        }
+        const ACC S_prev = __shfl_up_sync(0xFFFFFFFFu, Sc, 1);
+        const uint32_t next_r0 = __shfl_down_sync(0xFFFFFFFFu, r0, 1);
+        const int next_v = __shfl_down_sync(0xFFFFFFFFu, (int)started, 1);
+        // first run of a multi-run lane ends here
+        if (started && multi) fin(r0, A + (cont_prev ? S_prev : (ACC)0), d0, x0);
+        // last run: ends here unless the next lane or the next tile continues it
+        const bool next_cont = lane < 31 && next_v && next_r0 == rs;
+        const bool tile_cont = lane == 31 && (cur.r.w >> 31);
+        if (started && !next_cont && !tile_cont) fin(rs, Sc, dr, xr);
+        const int tc = __shfl_sync(0xFFFFFFFFu, (int)tile_cont, 31);
+        const ACC S31 = __shfl_sync(0xFFFFFFFFu, Sc, 31);
+        carry = tc ? S31 : (ACC)0;
+        cur = nxt;
+        nxt = nn;
+        v = vn;
+    }
+}
+
 template <typename W, bool MX, int CL>
 __device__ __forceinline__ void mid_level(const MidLevelDesc &d, cg::cluster_group &cl, double *sm,
-                                          double (*slot)[8], uint32_t *win, double *winx, double *wind) {
+                                          double (*slot)[8]) {
     typedef typename std::conditional<MX, float, double>::type ACC;
     const uint32_t n = d.n;
     const uint64_t m = d.m;
@@ -1845,6 +2021,8 @@ __device__ __forceinline__ void mid_level(const MidLevelDesc &d, cg::cluster_gro
     const uint64_t E0 = rp[R0], E1 = rp[R1];
     const uint32_t w0 = wk == 0 ? R0 : rows_at(rp, R0, R1, E0 + (E1 - E0) * wk / kMidWarps);
     const uint32_t w1 = wk + 1 == kMidWarps ? R1 : rows_at(rp, R0, R1, E0 + (E1 - E0) * (wk + 1) / kMidWarps);
+    uint4 *rows = d.rows + mid_tile0(rp[w0], rank * kMidWarps + wk) * 32;
+    mid_plan(rp, w0, w1, rows);
     // ---- phase 0: start vector (prolongated), weighted degrees, shift
     double p[4] = {0, 0, 0, 0};   // sum x, sum x d, sum d (normlap mean), max d
     bool empty_rows = false;
@@ -1915,9 +2093,7 @@ __device__ __forceinline__ void mid_level(const MidLevelDesc &d, cg::cluster_gro
             dst[i] = r;
             P[0] += r; P[1] += r * r; P[2] += ui * r; P[3] += ui; P[4] += ui * ui;
         };
-        if (w1 > w0)
-            warp_stream<true, MX, W, double, ACC>(rp, d.col, w, (const double *)src, m, d.vec_ok != 0, w0, w1,
-                                                  d.deg, win, winx, wind, fin);
+        mid_stream<MX, W, ACC>(rp, d.col, w, src, d.deg, m, d.vec_ok != 0, w0, w1, rows, fin);
         // rows without entries are not streamed: r = (gb - 0) u_i (u_i / 2
         // for the normalized walk)
         if (empty_rows && lane == 0)
@@ -1957,11 +2133,7 @@ __global__ void __launch_bounds__(kMidThreads, 1)
     cg::cluster_group cl = cg::this_cluster();
     __shared__ double sm[256];
     __shared__ double slot[2][8];
-    __shared__ uint32_t swin[kMidWarps][kWin + 3];
-    __shared__ double swinx[kMidWarps][kTile];
-    __shared__ double swind[kMidWarps][kTile];
     __shared__ uint32_t item;
-    const unsigned wk = threadIdx.x >> 5;
     while (true) {
         if (cl.block_rank() == 0 && threadIdx.x == 0) item = atomicAdd(next, 1u);
         cl.sync();
@@ -1978,11 +2150,11 @@ __global__ void __launch_bounds__(kMidThreads, 1)
             const MidLevelDesc &dsc = lev[ch.x + k];
             const unsigned long long t0 = global_ns();
             if (dsc.wbytes == 8) {
-                if (dsc.mixed) mid_level<unsigned long long, true, CL>(dsc, cl, sm, slot, swin[wk], swinx[wk], swind[wk]);
-                else mid_level<unsigned long long, false, CL>(dsc, cl, sm, slot, swin[wk], swinx[wk], swind[wk]);
+                if (dsc.mixed) mid_level<unsigned long long, true, CL>(dsc, cl, sm, slot);
+                else mid_level<unsigned long long, false, CL>(dsc, cl, sm, slot);
             } else {
-                if (dsc.mixed) mid_level<uint32_t, true, CL>(dsc, cl, sm, slot, swin[wk], swinx[wk], swind[wk]);
-                else mid_level<uint32_t, false, CL>(dsc, cl, sm, slot, swin[wk], swinx[wk], swind[wk]);
+                if (dsc.mixed) mid_level<uint32_t, true, CL>(dsc, cl, sm, slot);
+                else mid_level<uint32_t, false, CL>(dsc, cl, sm, slot);
             }
             // every block's part of the result is written before the next
             // level reads it, and every read of another block's slots is done
@@ -2918,13 +3090,14 @@ bool power_iter_mid_ok(const Level &L, const PowerIterOpts &o) {
     if (forced && *forced) return false;
     if (const char *e = getenv("SGPB_PI_MID"))
         if (atoi(e) == 0) return false;
-    if (L.n == 0 || power_iter_small_ok(L, o)) return false;
+    if (L.n == 0 || L.n > 0x7FFFFFFFu || power_iter_small_ok(L, o)) return false;   // mid_plan's bit 31
     if (!(L.wbytes == 0 || L.wbytes == 4 || L.wbytes == 8)) return false;
     if (!o.mid_limit && power_iter_slices_ok(L, o)) return false;
     return L.m + 8ull * L.n <= (o.mid_limit ? o.mid_limit : kMidCost);
 }
 
 int power_iter_mid_chains(Context &C, const std::vector<PIChain *> &chains, const PowerIterOpts &o) {
+    const int CLn = o.mid_blocks ? o.mid_blocks : kMidCTAs;   // blocks a cluster
     std::vector<MidLevelDesc> h;
     std::vector<std::pair<uint64_t, uint2>> order;   // (cost, chain) for largest-first
     for (PIChain *ch : chains) {
@@ -2951,6 +3124,7 @@ int power_iter_mid_chains(Context &C, const std::vector<PIChain *> &chains, cons
             SGPB_TRY(dalloc_t(C, &d.va, L.n));
             SGPB_TRY(dalloc_t(C, &d.vb, L.n));
             SGPB_TRY(dalloc_t(C, &d.deg, L.n));
+            SGPB_TRY(dalloc_t(C, &d.rows, mid_tiles(L.m, (uint32_t)CLn) * 32));
             d.tol = o.tol;
             d.iter_max = iter_budget(L.n, o);
             h.push_back(d);
@@ -2977,7 +3151,6 @@ int power_iter_mid_chains(Context &C, const std::vector<PIChain *> &chains, cons
     // as many clusters as fit at once (the queue balances the rest); CL
     // blocks a cluster: 8 for single partitions (latency of each level), 2
     // for batches (more hierarchies iterate at once)
-    const int CLn = o.mid_blocks ? o.mid_blocks : kMidCTAs;
     auto launch = [&](auto tag) -> int {
         constexpr int CL = decltype(tag)::value;
         const void *k = (const void *)k_power_iter_mid<CL>;
