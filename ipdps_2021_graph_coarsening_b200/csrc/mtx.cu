@@ -620,12 +620,13 @@ static bool par_pread(int fd, uint8_t *buf, size_t n, uint64_t off) {
     return ok.load();
 }
 
-// Bytes per ring slot for a transfer of `len` bytes: a power of two from 1 MiB
+// Bytes per ring slot for a transfer of `len` bytes: a power of two from 4 MiB
 // to `top`, about an eighth of the transfer, so that filling one slot overlaps
-// the copies of others (32 MB slots held a 13 MB text whole: the converter's
-// call 5.5 -> 5.2 ms, a context's first one, which pins the ring, 57 -> 9).
+// the copies of others.  The converter on a text of 24 MB: 5.55 ms with slots of
+// 32 MiB (one held the whole text), 5.4 from 1 MiB, 5.2 from 4, 5.15 from 8; a
+// context's first call, which pins the ring, 65, 20, 20 and 26 ms.
 static size_t stage_slot(uint64_t len, size_t top) {
-    size_t c = (size_t)1 << 20;
+    size_t c = (size_t)4 << 20;
     while (c < top && c * 8 < len) c *= 2;
     return c;
 }
