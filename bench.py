@@ -374,7 +374,9 @@ def gpu_arm(args, rank: int, ws: int, local: int, distmod):
     achieved = byts / (pi_ms / 1e3) / 1e9 if pi_ms > 0 else 0.0
     # DRAM bytes (read + write) of the step's power-iteration launches: the
     # ratio of measured DRAM bytes to algorithmic bytes from one ncu capture of
-    # the kernel on a smaller level, applied to this step's algorithmic bytes
+    # the CSR kernel on a smaller level, applied to this step's algorithmic
+    # bytes: an upper bound for row slices, which read about 2.2 bytes an entry
+    # of the largest coarse level where the model counts 8
     traffic = None
     tf = os.path.join(ROOT, "profiles", "power_iter_traffic.json")
     if os.path.exists(tf):
@@ -391,7 +393,7 @@ def gpu_arm(args, rank: int, ws: int, local: int, distmod):
                         "kernels": "HEC scan + map rounds + coarse builds of every level"}
     roofline_coarsen["frac"] = roofline_coarsen["achieved"] / peak
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "traffic": traffic, "kernel": "k_power_iter (+ k_power_iter_chains on the small levels)",
+                "traffic": traffic, "kernel": "k_pi_slices (+ k_power_iter on the finest level, k_power_iter_chains on the small levels)",
                 "peak_kind": peak_kind,
                 "kernel_ms_per_step": pi_ms, "algorithmic_bytes_per_step": byts,
                 "kernel_share_of_step": pi_ms / ms if ms else None}
