@@ -487,16 +487,17 @@ __global__ void __launch_bounds__(WARPS * 32) k_dedupe_radix(const uint32_t *__r
 // sparse; then each entry adds its weight at its place.  What bounds both
 // kernels is the chain of block barriers: five a bucket here, seven a digit pass
 // there.  Builds of an R-MAT 22 partition 12.1 -> 10.05 ms, of a weighted
-// Chung-Lu graph of 262,147 vertices 1.85 -> 1.44 ms.
-template <typename WI, int WARPS, int R>
+// Chung-Lu graph of 262,147 vertices 1.85 -> 1.44 ms.  The sums are as wide as
+// the coarse weights: 32-bit weights merge into 64-bit ones when the graph's
+// total does not fit 32 bits.
+template <typename WO, int WARPS, int R>
 struct BitsDedupeCfg {
-    typedef typename RadixDedupeCfg<WI, WARPS, R>::VT VT;
     static constexpr uint32_t kThreads = WARPS * 32, kCap = kThreads * R;
     // words from which a thread reads the bitmap through the summary
     static constexpr uint32_t kDirect = 8 * kThreads;
     static size_t smem(uint32_t nc) {
         const uint32_t nw = (nc + 31) / 32, ns = (nw + 31) / 32;
-        return (size_t)kCap * sizeof(VT) + 4 * ((size_t)nw + ns) + 2 * (size_t)nw;
+        return (size_t)kCap * sizeof(WO) + 4 * ((size_t)nw + ns) + 2 * (size_t)nw;
     }
 };
 
@@ -507,13 +508,12 @@ __global__ void __launch_bounds__(WARPS * 32) k_dedupe_bits(const uint32_t *__re
                                                             uint32_t *__restrict__ bdst, const WI *__restrict__ bw,
                                                             WO *__restrict__ tw, uint32_t *__restrict__ dcnt,
                                                             uint32_t nc) {
-    typedef BitsDedupeCfg<WI, WARPS, R> Cfg;
-    typedef typename Cfg::VT VT;
+    typedef BitsDedupeCfg<WO, WARPS, R> Cfg;
     constexpr uint32_t kThreads = Cfg::kThreads;
     __shared__ uint32_t s_tot[WARPS];
     extern __shared__ __align__(16) unsigned char rd_smem[];
     const uint32_t nw = (nc + 31) / 32, ns = (nw + 31) / 32;
-    VT *acc = reinterpret_cast<VT *>(rd_smem);
+    WO *acc = reinterpret_cast<WO *>(rd_smem);
     uint32_t *bits = reinterpret_cast<uint32_t *>(acc + Cfg::kCap);
     uint32_t *summary = bits + nw;
     uint16_t *pre = reinterpret_cast<uint16_t *>(summary + ns);   // at most kCap - 1 < 2^16
@@ -530,12 +530,12 @@ __global__ void __launch_bounds__(WARPS * 32) k_dedupe_bits(const uint32_t *__re
         const uint32_t c = list[k];
         const uint32_t b = boff[c], sz = boff[c + 1] - b;
         uint32_t key[R];
-        VT val[R];
+        WI val[R];
 #pragma unroll
         for (int r = 0; r < R; r++) {
             const uint32_t q = r * kThreads + threadIdx.x;
             key[r] = q < sz ? bdst[b + q] : kSentinel;
-            val[r] = q < sz ? (bw ? (VT)bw[b + q] : (VT)1) : (VT)0;
+            val[r] = q < sz ? (bw ? bw[b + q] : (WI)1) : (WI)0;
         }
 #pragma unroll
         for (int r = 0; r < R; r++)
@@ -584,12 +584,12 @@ __global__ void __launch_bounds__(WARPS * 32) k_dedupe_bits(const uint32_t *__re
             if (key[r] != kSentinel) {
                 const uint32_t j = key[r] >> 5;
                 const uint32_t pos = pre[j] + __popc(bits[j] & ((1u << (key[r] & 31)) - 1u));
-                atomicAdd(acc + pos, val[r]);
+                atomicAdd(acc + pos, (WO)val[r]);
                 bdst[b + pos] = key[r];   // equal destinations write the same value
             }
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < total; i += kThreads) {
-            tw[b + i] = (WO)acc[i];
+            tw[b + i] = acc[i];
             acc[i] = 0;
         }
 #pragma unroll
@@ -616,7 +616,7 @@ static int dedupe_tier(Context &C, uint32_t nc, int passes, uint32_t per_sm, con
                        const uint32_t *count, const uint32_t *boff, uint32_t *bdst, const WI *bw, WO *tw,
                        uint32_t *dcnt) {
     constexpr uint32_t T = WARPS * 32;
-    const size_t smem = BitsDedupeCfg<WI, WARPS, R>::smem(nc);
+    const size_t smem = BitsDedupeCfg<WO, WARPS, R>::smem(nc);
     const uint32_t fit = (uint32_t)((C.smem_optin + 1024) / (smem + 1024 + 64));
     if (fit * T >= kBitsMinThreads) {
         const uint32_t g = fit < per_sm ? fit : per_sm;

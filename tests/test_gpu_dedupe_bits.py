@@ -5,6 +5,8 @@ the oracle's build."""
 import numpy as np
 import pytest
 
+from ipdps_2021_graph_coarsening_b200 import graphs as G
+from ipdps_2021_graph_coarsening_b200.api import PCG32
 from oracle import bindings as O
 from tests.test_gpu_parity import dev_u32, host_u32, host_u64
 
@@ -77,3 +79,38 @@ def test_bitmap_dedupe(partitioner, nc, width):
     got = host_u32(crp), host_u32(ccol), (host_u64(cw) if width == 8 else host_u32(cw)).astype(np.uint64)
     for a, b in zip(got, want):
         assert np.array_equal(a, b)
+
+
+# 32-bit weights into 64-bit sums, as a graph whose total needs 64 bits is
+# built: weights near 2^32, so that every pair of equal destinations sums to
+# more than 32 bits; buckets of every tier, on both sides of the radix rule
+@pytest.mark.parametrize("nc", [33, 1025, 16385, 190000, 420001, 1200001])
+def test_sums_wider_than_weights(partitioner, nc):
+    rp, col, vc = level(nc, nc + 1, SIZES + DENSE)
+    w = np.random.default_rng(2).integers((1 << 32) - 1000, 1 << 32, col.size).astype(np.uint64)
+    want = O.build_coarse(rp, col, w, vc, nc)
+    assert want[2].max() >= 1 << 32
+    crp, ccol, cw = partitioner.build_coarse(dev_u32(rp), dev_u32(col), dev_u32(w.astype(np.uint32)), dev_u32(vc), nc,
+                                             8)
+    for a, b in zip((host_u32(crp), host_u32(ccol), host_u64(cw)), want):
+        assert np.array_equal(a, b)
+
+
+def test_hierarchy_of_a_total_above_32_bits(partitioner):
+    g = G.rmat(13, seed=5)
+    rows = np.repeat(np.arange(g.n), np.diff(g.row_ptr.astype(np.int64)))
+    lo, hi = np.minimum(rows, g.col).astype(np.uint64), np.maximum(rows, g.col).astype(np.uint64)
+    w = ((1 << 32) - 1 - (lo * 31 + hi * 17) % 1000).astype(np.uint32)   # symmetric
+    seed = 0x853C49E6748FEA9B
+    h = partitioner.generate_coarse_graphs(G.CSR(g.row_ptr, g.col, w), 50, PCG32(seed))
+    o = O.partition_graph(g.row_ptr, g.col, w, cutoff=50, rng_state=seed)
+    assert len(h) == len(o["level_n"]) > 2
+    rp, col, cw = g.row_ptr, g.col, w.astype(np.uint64)
+    for l in range(1, len(h)):
+        vc = host_u32(h.level(l - 1)["vcmap"])
+        lv = h.level(l)
+        assert lv["n"] == o["level_n"][l] and lv["wbytes"] == 8
+        rp, col, cw = O.build_coarse(rp, col, cw, vc, lv["n"])
+        assert np.array_equal(host_u32(lv["row_ptr"]), rp) and np.array_equal(host_u32(lv["col"]), col)
+        assert np.array_equal(host_u64(lv["w"]), cw)
+    h.free()
