@@ -206,9 +206,9 @@ __global__ void k_normalize_guess(double *x, uint32_t n) {
 
 // eigensolve_kokkos.h:1493-1595 without FM, in two parts so that a batch can
 // run the small and mid-size levels of all its hierarchies in two launches.
-// eigen_begin draws and normalises the coarsest guess and plans the chain of
-// small levels from the coarsest one up, then the chain of mid-size levels
-// above it (the levels stay in `levels`, which must not be resized
+// eigen_begin draws and normalises the coarsest guess; eigen_plan plans the
+// chain of small levels from the coarsest one up, then the chain of mid-size
+// levels above it (the levels stay in `levels`, which must not be resized
 // afterwards); the chains run through power_iter_chains and
 // power_iter_mid_chains (run_chains); eigen_finish records their results and
 // iterates the remaining levels, prolongating down.
@@ -217,6 +217,8 @@ struct EigenState {
     PIChain chain;   // small levels
     PIChain mid;     // mid-size levels, starting from the small chain's result
 };
+
+static int eigen_plan(Context &C, std::vector<Level> &levels, const PowerIterOpts &o, EigenState *E);
 
 static int eigen_begin(Context &C, std::vector<Level> &levels, uint64_t *rng_state, uint64_t rng_inc,
                        const PowerIterOpts &o, EigenState *E) {
@@ -231,7 +233,12 @@ static int eigen_begin(Context &C, std::vector<Level> &levels, uint64_t *rng_sta
     k_normalize_guess<<<1, 256, 0, C.stream>>>(x, gn);
     C.kernel_launches++;
     E->x0 = x;
-    E->chain.x0 = x;
+    return eigen_plan(C, levels, o, E);
+}
+
+static int eigen_plan(Context &C, std::vector<Level> &levels, const PowerIterOpts &o, EigenState *E) {
+    const int L = (int)levels.size();
+    E->chain.x0 = E->x0;
     E->chain.lev.clear();
     int l = L - 1;
     for (; l >= 0 && power_iter_small_ok(levels[l], o); l--) {
@@ -241,7 +248,7 @@ static int eigen_begin(Context &C, std::vector<Level> &levels, uint64_t *rng_sta
         SGPB_TRY(dalloc_t(C, &cl.x_out, levels[l].n));
         E->chain.lev.push_back(cl);
     }
-    E->mid.x0 = E->chain.lev.empty() ? x : E->chain.lev.back().x_out;
+    E->mid.x0 = E->chain.lev.empty() ? E->x0 : E->chain.lev.back().x_out;
     E->mid.lev.clear();
     for (; l >= 0 && power_iter_mid_ok(levels[l], o); l--) {
         PIChainLevel cl;
@@ -265,9 +272,11 @@ static int run_chains(Context &C, const std::vector<EigenState *> &es, const Pow
     return power_iter_mid_chains(C, mid, o);
 }
 
+// *close: a level's iteration stopped within kStopMargin of tol
 static int eigen_finish(Context &C, std::vector<Level> &levels, const PowerIterOpts &o, const EigenState &E,
-                        double **evec_out, PowerIterResult *finest) {
+                        double **evec_out, PowerIterResult *finest, bool *close) {
     const int L = (int)levels.size();
+    *close = false;
     std::vector<const PIChainLevel *> done;   // chain levels from the coarsest one down
     for (const PIChainLevel &cl : E.chain.lev) done.push_back(&cl);
     for (const PIChainLevel &cl : E.mid.lev) done.push_back(&cl);
@@ -280,6 +289,7 @@ static int eigen_finish(Context &C, std::vector<Level> &levels, const PowerIterO
         lv.pi_capped = r.capped;
         lv.pi_dot = r.dot;
         lv.pi_lambda = r.lambda;
+        *close |= r.close;
         if (L - 1 - k == 0) {
             *finest = r;
             SGPB_TRY(level_residual(C, lv, done[k]->x_out, o.normlap, finest));
@@ -303,6 +313,7 @@ static int eigen_finish(Context &C, std::vector<Level> &levels, const PowerIterO
         lv.pi_capped = r.capped;
         lv.pi_dot = r.dot;
         lv.pi_lambda = r.lambda;
+        *close |= r.close;
         if (l == 0) *finest = r;
         xin = xo;
     }
@@ -310,12 +321,27 @@ static int eigen_finish(Context &C, std::vector<Level> &levels, const PowerIterO
     return SGP_B200_OK;
 }
 
+// the whole solve from the same guess in the plain order of sums
+static int eigen_again(Context &C, std::vector<Level> &levels, const PowerIterOpts &o, const EigenState &E,
+                       double **evec_out, PowerIterResult *finest) {
+    PowerIterOpts op = o;
+    op.plain = 1;
+    EigenState Ep;
+    Ep.x0 = E.x0;
+    SGPB_TRY(eigen_plan(C, levels, op, &Ep));
+    SGPB_TRY(run_chains(C, {&Ep}, op));
+    bool close;
+    return eigen_finish(C, levels, op, Ep, evec_out, finest, &close);
+}
+
 static int eigensolve(Context &C, std::vector<Level> &levels, uint64_t *rng_state, uint64_t rng_inc,
                       const PowerIterOpts &o, double **evec_out, PowerIterResult *finest) {
     EigenState E;
     SGPB_TRY(eigen_begin(C, levels, rng_state, rng_inc, o, &E));
     SGPB_TRY(run_chains(C, {&E}, o));
-    return eigen_finish(C, levels, o, E, evec_out, finest);
+    bool close;
+    SGPB_TRY(eigen_finish(C, levels, o, E, evec_out, finest, &close));
+    return close ? eigen_again(C, levels, o, E, evec_out, finest) : SGP_B200_OK;
 }
 
 static float ev_ms(cudaEvent_t a, cudaEvent_t b) {
@@ -373,11 +399,20 @@ static int partition_end(Context &C, const sgp_b200_options_t *opt, sgp_b200_res
     std::vector<Level> &levels = S.levels;
     double *evec = nullptr;
     PowerIterResult fin;
-    SGPB_TRY(eigen_finish(C, levels, S.po, S.es, &evec, &fin));
-    SGPB_CUDA(cudaEventRecord(ev[3], C.stream));
+    bool close = false, tie = false;
+    const bool plain = pi_plain(S.po);
+    SGPB_TRY(eigen_finish(C, levels, S.po, S.es, &evec, &fin, &close));
     uint64_t cut = 0;
     uint32_t p0 = 0;
-    SGPB_TRY(split_level(C, levels[0], evec, opt->perc_imbalance, part_d, &cut, &p0));
+    if (!close) {
+        SGPB_CUDA(cudaEventRecord(ev[3], C.stream));
+        SGPB_TRY(split_level(C, levels[0], evec, opt->perc_imbalance, part_d, &cut, &p0, plain ? nullptr : &tie));
+    }
+    if (close || tie) {   // not certain to be the plain order's partition
+        SGPB_TRY(eigen_again(C, levels, S.po, S.es, &evec, &fin));
+        SGPB_CUDA(cudaEventRecord(ev[3], C.stream));
+        SGPB_TRY(split_level(C, levels[0], evec, opt->perc_imbalance, part_d, &cut, &p0));
+    }
     res->ls_swaps = 0;
     if (opt->local_search_alg) {
         // the part-0 size is the reference's curr_split when the split's
@@ -948,8 +983,13 @@ int sgp_b200_power_iter(sgp_b200_ctx_t *x, uint32_t n, const uint32_t *rp, const
     o.tol = tol;
     o.iter_cap = iter_cap;
     o.mixed = mixed;
+    o.plain = x_in == x_out;   // the result may be needed in the other order, from the same vector
     PowerIterResult r;
     if (rc == SGP_B200_OK) rc = power_iter_level(*C, L, x_in, vcmap, x_out, o, &r, residual != nullptr);
+    if (rc == SGP_B200_OK && r.close) {
+        o.plain = 1;
+        rc = power_iter_level(*C, L, x_in, vcmap, x_out, o, &r, residual != nullptr);
+    }
     if (rc == SGP_B200_OK) {
         if (niter) *niter = r.niter;
         if (lambda) *lambda = r.lambda;

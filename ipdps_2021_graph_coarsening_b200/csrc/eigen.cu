@@ -95,6 +95,7 @@ struct PIArgs {
     const void *pw;               // weights (same width as w), null when unweighted
     void *yacc;                   // [n] row sums over the panels so far (iterate type)
     uint32_t *err;                // staged rows (mode 7): set when a bulk copy did not complete in time
+    double *margin;               // least distance of an iteration's change from tol, 0 if r cancelled (null: not kept)
 };
 
 // dynamic shared memory for the iterate cache, per block (two blocks per SM)
@@ -1252,6 +1253,8 @@ __global__ void __launch_bounds__(kPIThreads, 2) k_power_iter(PIArgs a) {
         dot = (S[2] - mu_n * S[3]) * inv_nu_n;
         niter++;
         const double delta = fabs(dot - last);
+        if (a.margin && blockIdx.x == 0 && threadIdx.x == 0)
+            *a.margin = nsq > kCancel * gb * gb ? fmin(*a.margin, fabs(delta - a.tol)) : 0.0;
         if (STAGED && *(volatile uint32_t *)a.err) {
             // a bulk copy did not complete: every block leaves here (the flag
             // was set before the barrier), the host reports the error
@@ -1555,6 +1558,7 @@ __device__ __noinline__ void small_level_rows(const PIArgs &a) {
     if (tid == 0) sm[128] = q[0];
     __syncthreads();
     double inv_nu = 1.0 / sqrt(sm[128]);
+    double margin = sm[128] > kCancel * (double)n * mu * mu ? 1e300 : 0.0;   // PIArgs::margin
     // lanes per row: the least of (rows after the first of a thread) * mean +
     // longest row, per lane, and fixed prices of a row, a butterfly step (three
     // entries' time) and the barrier of several warps
@@ -1592,6 +1596,7 @@ __device__ __noinline__ void small_level_rows(const PIArgs &a) {
         const double d0 = one ? deg[row0] : 0.0;
         const uint32_t r0 = one ? row0 : 0u, j0 = b0 + g + (kHeld << lg);
         const double rn = 1.0 / (double)n;
+        const double r_min = kCancel * gb * gb;
         double dot = 0, last = 0;
         uint64_t niter = 0;
         double *src = xa, *dst = xb;
@@ -1671,11 +1676,13 @@ __device__ __noinline__ void small_level_rows(const PIArgs &a) {
                 buf ^= 1;
             }
             const double mu_n = A * rn;
-            const double inv_n = rsqrt(B - mu_n * A);
+            const double nsq = B - mu_n * A;
+            const double inv_n = rsqrt(nsq);
             last = dot;
             dot = s_ur * inv_n;
             niter++;
             const double delta = fabs(dot - last);
+            margin = nsq > r_min ? fmin(margin, fabs(delta - a.tol)) : 0.0;
             if (!(delta > a.tol && niter < a.iter_max)) break;
             mu = mu_n;
             inv_nu = inv_n;
@@ -1701,6 +1708,7 @@ __device__ __noinline__ void small_level_rows(const PIArgs &a) {
             a.res[3] = (gb * t - s_ur) / t;
             a.res[4] = niter >= a.iter_max ? 1.0 : 0.0;
             a.res[5] = 0.0;
+            a.res[7] = margin;
         }
     }
 }
@@ -1790,7 +1798,7 @@ struct MidLevelDesc {
     uint4 *rows;             // [mid_tiles(m, blocks)][32] rows of each lane's entries (mid_plan)
     double tol;
     uint64_t iter_max;
-    double *res;             // [0] niter [1] dot [2] gb [3] lambda [4] capped [6] ms
+    double *res;             // [0] niter [1] dot [2] gb [3] lambda [4] capped [6] ms [7] margin (PIArgs)
 };
 
 // Tiles of kTile entries from the multiple of four at or below a warp's first
@@ -2083,6 +2091,7 @@ __device__ __forceinline__ void mid_level(const MidLevelDesc &d, cg::cluster_gro
     double inv_nu = 1.0 / sqrt(q[0]);
     // ---- iterations
     double dot = 0, last = 1;
+    double margin = q[0] > kCancel * (double)n * mu * mu ? 1e300 : 0.0;   // PIArgs::margin
     uint64_t niter = 0;
     double *src = d.va, *dst = d.vb;
     while (true) {
@@ -2108,6 +2117,7 @@ __device__ __forceinline__ void mid_level(const MidLevelDesc &d, cg::cluster_gro
         dot = (P[2] - mu_n * P[3]) * inv_nu_n;
         niter++;
         const double delta = fabs(dot - last);
+        margin = nsq > kCancel * gb * gb ? fmin(margin, fabs(delta - d.tol)) : 0.0;
         if (!(delta > d.tol && niter < d.iter_max)) {
             for (uint32_t i = R0 + threadIdx.x; i < R1; i += blockDim.x) d.out[i] = (src[i] - mu) * inv_nu;
             if (rank == 0 && threadIdx.x == 0) {
@@ -2116,6 +2126,7 @@ __device__ __forceinline__ void mid_level(const MidLevelDesc &d, cg::cluster_gro
                 d.res[2] = gb;
                 d.res[3] = d.normlap ? 2.0 * (1.0 - P[2] / P[4]) : (gb * P[4] - P[2]) / P[4];
                 d.res[4] = niter >= d.iter_max ? 1.0 : 0.0;
+                d.res[7] = margin;
             }
             break;
         }
@@ -2569,7 +2580,7 @@ static int launch_pi(Context &C, PIArgs &a, uint32_t grid, int mode) {
 // levels, else the cooperative kernel (column panels when a layout is given).
 // mixed: FP32 edge-difference arithmetic (never with panels or small levels).
 static int run_pi(Context &C, const Level &L, PIArgs a, bool mixed, const PanelLayout *panels, double *res_d,
-                  double res_h[7], float *ms, uint32_t grid, int mode) {
+                  double res_h[8], float *ms, uint32_t grid, int mode) {
     a.res = res_d;
     a.P = 0;
     if (panels) {
@@ -2620,9 +2631,9 @@ static int run_pi(Context &C, const Level &L, PIArgs a, bool mixed, const PanelL
     cudaEventRecord(e1, C.stream);
     if (rc != SGP_B200_OK) { cudaEventDestroy(e0); cudaEventDestroy(e1); return rc; }
     SGPB_CUDA(cudaGetLastError());
-    SGPB_CUDA(cudaMemcpyAsync(C.h_pinned, res_d, 7 * sizeof(double), cudaMemcpyDeviceToHost, C.stream));
+    SGPB_CUDA(cudaMemcpyAsync(C.h_pinned, res_d, 8 * sizeof(double), cudaMemcpyDeviceToHost, C.stream));
     SGPB_CUDA(cudaStreamSynchronize(C.stream));
-    memcpy(res_h, C.h_pinned, 7 * sizeof(double));
+    memcpy(res_h, C.h_pinned, 8 * sizeof(double));
     if (!small && ((const double *)C.h_pinned)[5] != 0.0) {
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
@@ -2756,7 +2767,7 @@ static int autotune_level(Context &C, const Level &L, const PIArgs &a0, bool mix
         a.out = scratch;
         a.iter_max = kTuneIters;
         a.tol = -1.0;   // run exactly kTuneIters iterations
-        double rh[7];
+        double rh[8];
         float k = 0;
         SGPB_TRY(run_pi(C, L, a, mixed, nullptr, res_d, rh, &k, pi_grid(C, L.n, L.m, c.units), c.mode));
         *ms = k;
@@ -2918,7 +2929,11 @@ int power_iter_level(Context &C, const Level &Lin, const double *x_in, const uin
     a.tol = o.tol;
     double *res_d;
     SGPB_TRY(dalloc_t(C, &res_d, 8));
-    double rh[7];
+    if (!pi_plain(o)) {
+        a.margin = res_d + 7;
+        SGPB_CUDA(cudaMemsetAsync(a.margin, 0x7F, sizeof(double), C.stream));   // 1.4e306
+    }
+    double rh[8];
     float kms = 0;
     PanelLayout panels;
     if (want_panels) SGPB_TRY(build_panels(C, L, a.heavy_T, sizeof(double), &panels));
@@ -2929,6 +2944,7 @@ int power_iter_level(Context &C, const Level &Lin, const double *x_in, const uin
         // with, the dot product before it carried over
         SGPB_TRY(power_iter_slices(C, Lin, x_out, nullptr, x_out, o, imax, kProbeIters - 1, rh[6], res, &fits));
         if (fits) {
+            res->close = res->close || rh[7] < kStopMargin;
             res->kernel_ms += kms;
             if (want_residual) SGPB_TRY(level_residual(C, Lin, x_out, o.normlap, res));
             return SGP_B200_OK;
@@ -2944,6 +2960,7 @@ int power_iter_level(Context &C, const Level &Lin, const double *x_in, const uin
     res->lambda = rh[3];
     res->capped = rh[4] != 0.0;
     res->resid = 0;
+    res->close = a.margin && rh[7] < kStopMargin;
     res->kernel_ms = kms;
     // the result is in the level's own numbering: use the level itself
     if (want_residual) SGPB_TRY(level_residual(C, Lin, x_out, o.normlap, res));
@@ -2996,6 +3013,14 @@ int level_residual(Context &C, const Level &L, const double *x, int normlap, Pow
     return SGP_B200_OK;
 }
 
+bool pi_plain(const PowerIterOpts &o) {
+    if (o.plain || o.mixed || o.normlap || (o.tol >= 0 && o.tol < kPlainTol)) return true;
+    if (const char *e = getenv("SGPB_PI_MODE"))
+        if (*e) return true;
+    const char *e = getenv("SGPB_PI_SLICES");
+    return e && atoi(e) == 0;
+}
+
 bool power_iter_small_ok(const Level &L, const PowerIterOpts &o) {
     const char *forced = getenv("SGPB_PI_MODE");
     if (forced && *forced) return false;
@@ -3030,10 +3055,7 @@ int power_iter_chains(Context &C, const std::vector<PIChain *> &chains, const Po
             d.a.iter_max = iter_budget(L.n, o);
             d.a.normlap = o.normlap;
             d.wbytes = L.wbytes;
-            // mixed runs and the normalized walk keep small_level's order of
-            // sums: the FP32 differences of a mixed run's larger levels, and
-            // the walk without deflation, amplify any other rounding
-            d.rows = !o.mixed && !o.normlap;
+            d.rows = !pi_plain(o);
             h.push_back(d);
             cost += L.m + 8ull * L.n;
             const size_t b = L.wbytes == 8 ? small_level_bytes<unsigned long long, double>(L.n, L.m, L.w != nullptr)
@@ -3079,6 +3101,7 @@ int power_iter_chains(Context &C, const std::vector<PIChain *> &chains, const Po
             cl.res.gb = r[2];
             cl.res.lambda = r[3];
             cl.res.capped = r[4] != 0.0;
+            cl.res.close = !pi_plain(o) && r[7] < kStopMargin;
             cl.res.kernel_ms = (float)r[6];
         }
     }
@@ -3201,6 +3224,7 @@ int power_iter_mid_chains(Context &C, const std::vector<PIChain *> &chains, cons
             cl.res.gb = r[2];
             cl.res.lambda = r[3];
             cl.res.capped = r[4] != 0.0;
+            cl.res.close = !pi_plain(o) && r[7] < kStopMargin;
             cl.res.kernel_ms = (float)r[6];
         }
     }

@@ -170,6 +170,7 @@ struct PowerIterOpts {
     int allow_relabel = 1;   // skewed levels may iterate on a hub-first relabelled copy
     int normlap = 0;         // refine_alg 1: normalized-Laplacian (lazy random walk) iteration
     int probe = 0;           // 1: the level may stop after a few iterations (the finest one)
+    int plain = 0;           // 1: the plain order of sums (see pi_plain)
     uint64_t mid_limit = 0;  // largest cost (m + 8n) of a level on the cluster kernel; 0 = the rule:
                              // 2^17, and none of the levels that run on row slices
     int mid_blocks = 0;       // blocks per cluster of the cluster kernel (2 or 8); 0 = 8
@@ -179,7 +180,34 @@ struct PowerIterResult {
     int capped = 0;
     double dot = 0, gb = 0, lambda = 0, resid = 0;
     float kernel_ms = 0;     // cooperative-kernel time (CUDA events)
+    bool close = false;      // a stopping decision lay within kStopMargin of tol, or an iterate cancelled
 };
+// Two orders of sums.  The plain one (k_power_iter, small_level, the cluster
+// kernel) defines the partitions of this library; row slices and
+// small_level_rows are faster and add in another order, so their vectors differ
+// from it by rounding: at most 6.4e-15 / sqrt(n) near the median over 240 graphs
+// of every family the tests use, and 216 of R-MAT 22.  A partition takes the
+// fast order and is certified afterwards: it is the plain order's if no other
+// vertex lies within kTieGap / sqrt(n) of the median (split_level), every
+// iteration's change was further than kStopMargin from tol, and no iterate
+// cancelled (kCancel in pi_common.cuh); otherwise the plain order decides.
+// Gaps are 2e-9 / sqrt(n) and more or about zero: leaves of one aggregate are
+// equal in exact arithmetic, and which of them come first is the plain order's
+// rounding (the median falls among such vertices in 46 of 280 R-MAT 22 graphs,
+// in 15 of 120 of R-MAT 13..19, 3 of 120 3D meshes, none of 360 others).  Dot
+// products of the two orders, near 1, differ by a few units of 1.1e-16; with
+// twice this margin 27 of 720 graphs were repeated for it, while none of 1,136
+// graphs had another number of iterations.
+constexpr double kTieGap = 1e-12;
+constexpr double kStopMargin = 1e-15;
+// below this tolerance an iteration's change comes near the rounding of the dot
+// products, so that the number of iterations is the rounding's
+constexpr double kPlainTol = 1e-11;
+// whether levels run in the plain order: asked for, a tolerance below
+// kPlainTol, mixed precision (whose FP32 differences amplify any other
+// rounding), the normalized walk (no deflation in its loop), a forced kernel
+// (SGPB_PI_MODE), or SGPB_PI_SLICES=0
+bool pi_plain(const PowerIterOpts &o);
 // x_in: coarse vector (prolongated through vcmap when vcmap != null) or the
 // initial vector; x_out: n doubles (may alias nothing).
 int power_iter_level(Context &C, const Level &L, const double *x_in, const uint32_t *vcmap,
@@ -220,8 +248,9 @@ int power_iter_chains(Context &C, const std::vector<PIChain *> &chains, const Po
 // first, one cluster per chain at a time, in one launch.
 bool power_iter_mid_ok(const Level &L, const PowerIterOpts &o);
 int power_iter_mid_chains(Context &C, const std::vector<PIChain *> &chains, const PowerIterOpts &o);
+// close (if not null): another vertex's value lies within kTieGap / sqrt(n) of the median's
 int split_level(Context &C, const Level &L, const double *evec, int perc_imbalance, uint32_t *part,
-                uint64_t *edgecut, uint32_t *n_part0);
+                uint64_t *edgecut, uint32_t *n_part0, bool *close = nullptr);
 int edge_cut_device(Context &C, const Level &L, const uint32_t *part, uint64_t *edgecut);
 // bitmap of a part array (bits.cuh); the rows of more than kLongRow entries in
 // any order, their number added to *nlong

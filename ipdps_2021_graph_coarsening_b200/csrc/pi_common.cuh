@@ -23,6 +23,12 @@ __device__ __forceinline__ double next_value(int normlap, double gb, double mu, 
     }
 }
 
+// An iterate whose norm is this much smaller than the terms it is the sum of
+// has lost as much of its precision, and the order of its sums shows: a start
+// vector against its mean (|x - mean|^2 / (n mean^2)), r against the shift
+// (|r|^2 / gb^2 with |u| = 1; two vertices joined by an edge have r = 0).
+constexpr double kCancel = 1e-6;
+
 // Sum of three values over a warp, packed: value k of the warp ends up in
 // lanes with (lane & 3) == k (k < 3).  6 double shuffles instead of 15.
 __device__ __forceinline__ double warp_sum3(double a, double b, double c) {

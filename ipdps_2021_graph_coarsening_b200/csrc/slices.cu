@@ -94,6 +94,7 @@ struct SliceArgs {
     double tol;
     uint64_t iter_max;
     double *res;                  // [0] niter [1] dot [2] gb [3] lambda [4] capped [5] barrier gave up
+                                  // [7] least distance of an iteration's change from tol, 0 if an iterate cancelled
     // continued run: iterations already done and the last dot product but one
     uint64_t iter0;
     double dot0;
@@ -388,6 +389,7 @@ __global__ void __launch_bounds__(slice_threads(FORM, WB), 1) k_pi_slices(SliceA
     __shared__ double sm[kSliceWarps][kSumK];
     __shared__ double s_sum[4];
     __shared__ double s_it[3];   // mean, 1 / norm and dot product of the last iteration
+    __shared__ double s_margin;  // res[7]
     __shared__ uint32_t s_ok;
     const uint32_t n = a.n;
     const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -395,6 +397,7 @@ __global__ void __launch_bounds__(slice_threads(FORM, WB), 1) k_pi_slices(SliceA
     __shared__ __align__(8) uint64_t s_mbar;
     GridBar bar{a.bar, a.err, 0};
     PanelCopy panel{&s_mbar, 0};
+    if (threadIdx.x == 0) s_margin = 1e300;
     if (COPY) panel.init();   // seen by the block behind the start vector's barriers
     double *part0 = a.partials, *part1 = a.partials + 4 * (size_t)gridDim.x;
     if (COPY && threadIdx.x < kBanks) xs[kSlicePW + threadIdx.x] = 0.0;
@@ -467,6 +470,7 @@ __global__ void __launch_bounds__(slice_threads(FORM, WB), 1) k_pi_slices(SliceA
         if (wid == 0) grid_sum3(part1, s_sum);
         __syncthreads();
         inv_nu = 1.0 / sqrt(s_sum[0]);
+        if (threadIdx.x == 0 && !(s_sum[0] > kCancel * (double)n * mu * mu)) s_margin = 0;
         __syncthreads();
     }
     // ---- iterations
@@ -510,6 +514,7 @@ __global__ void __launch_bounds__(slice_threads(FORM, WB), 1) k_pi_slices(SliceA
                 s_it[0] = m;
                 s_it[1] = inv;
                 s_it[2] = s_sum[2] * inv;
+                s_margin = nsq > kCancel * gb * gb ? fmin(s_margin, fabs(fabs(s_it[2] - dot) - a.tol)) : 0.0;
             }
         }
         if (COPY && (!PANELS || U0 < U1))
@@ -546,6 +551,7 @@ __global__ void __launch_bounds__(slice_threads(FORM, WB), 1) k_pi_slices(SliceA
                         a.res[3] = (gb * S5 - s_ur) / S5;
                         a.res[4] = niter >= a.iter_max ? 1.0 : 0.0;
                         a.res[5] = 0.0;
+                        a.res[7] = s_margin;
                     }
                 }
                 return;
@@ -1148,13 +1154,7 @@ static SliceForm slice_form(uint32_t n, uint64_t m, bool skew, uint64_t tail) {
 }
 
 bool power_iter_slices_ok(const Level &L, const PowerIterOpts &o) {
-    if (const char *e = getenv("SGPB_PI_MODE"))
-        if (*e) return false;
-    if (const char *e = getenv("SGPB_PI_SLICES"))
-        if (atoi(e) == 0) return false;
-    // the normalized walk has no deflation in its loop: what it ends on depends
-    // on the rounding of the main kernel's sums
-    if (o.normlap || (o.mixed && L.n >= 4096)) return false;
+    if (pi_plain(o)) return false;
     if (L.n == 0 || L.m == 0 || L.n > 0x7FFFFFFFu) return false;
     return L.wbytes == 0 || L.wbytes == 4 || L.wbytes == 8;
 }
@@ -1411,11 +1411,11 @@ static int slices_run(Context &C, const Level &L, const double *x_in, const uint
     SGPB_CUDA(cudaLaunchCooperativeKernel(k, dim3(grid), dim3((unsigned)threads), args, dyn, C.stream));
     C.kernel_launches++;
     SGPB_CUDA(cudaEventRecord(ev[1], C.stream));
-    SGPB_CUDA(cudaMemcpyAsync(C.h_pinned, res_d, 6 * sizeof(double), cudaMemcpyDeviceToHost, C.stream));
-    SGPB_CUDA(cudaMemcpyAsync((double *)C.h_pinned + 6, a.err, 4, cudaMemcpyDeviceToHost, C.stream));
+    SGPB_CUDA(cudaMemcpyAsync(C.h_pinned, res_d, 8 * sizeof(double), cudaMemcpyDeviceToHost, C.stream));
+    SGPB_CUDA(cudaMemcpyAsync((double *)C.h_pinned + 8, a.err, 4, cudaMemcpyDeviceToHost, C.stream));
     SGPB_CUDA(cudaStreamSynchronize(C.stream));
     const double *r = (const double *)C.h_pinned;
-    if (*(const uint32_t *)(r + 6)) {
+    if (*(const uint32_t *)(r + 8)) {
         set_error("power iteration: a grid barrier did not complete within its wait limit");
         return SGP_B200_ERR_DEVICE;
     }
@@ -1425,6 +1425,7 @@ static int slices_run(Context &C, const Level &L, const double *x_in, const uint
     res->lambda = r[3];
     res->capped = r[4] != 0.0;
     res->resid = 0;
+    res->close = r[7] < kStopMargin;
     float t = 0;
     cudaEventElapsedTime(&t, ev[0], ev[1]);
     res->kernel_ms = t;

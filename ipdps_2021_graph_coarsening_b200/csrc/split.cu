@@ -48,13 +48,23 @@ struct SplitArgs {
     uint32_t *longs;       // rows of more than kLongRow entries, in any order
     uint32_t *part;
     unsigned long long *out;        // [0] edgecut [1] part0 size [2] threshold index [3] directed cross entries
+    double gap;                     // >= 0: out[4..7] too, see below
 };
+// The certificate of a split (gap >= 0): out[4] largest key below the
+// threshold's, out[5] least key of the vertices behind the threshold, out[6]
+// the threshold's key, out[7] whether a vertex on the other side of a decision
+// lies within gap of the threshold.
+constexpr size_t kSplitOutWords = 8;
 constexpr size_t kSplitHistWords = 3 * kSelBins + 2;
 
 __device__ __forceinline__ unsigned long long order_key(double x) {
     if (x == 0.0) x = 0.0;   // -0.0 == +0.0 in the reference's comparator
     unsigned long long b = (unsigned long long)__double_as_longlong(x);
     return (b & 0x8000000000000000ull) ? ~b : (b | 0x8000000000000000ull);
+}
+
+__device__ __forceinline__ double key_value(unsigned long long k) {
+    return __longlong_as_double((long long)((k >> 63) ? k & ~(1ull << 63) : ~k));
 }
 
 __global__ void __launch_bounds__(kSplitThreads) k_split(SplitArgs a) {
@@ -68,6 +78,10 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(SplitArgs a) {
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
     uint32_t *ncand = a.hist + 3 * kSelBins, *nlong = ncand + 1;
+    if (a.gap >= 0 && tid == 0) {   // next used behind a grid barrier
+        a.out[4] = 0;
+        a.out[5] = ~0ull;
+    }
     // select: prefix over (key:64, index:32), digits MSB first: the key in five
     // of 11 bits and one of 9, the index in two of 11 and one of 10
     unsigned long long kpre = 0;   // selected key bits so far
@@ -168,6 +182,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(SplitArgs a) {
         break;
     }
     // assign parts; a.k elements precede the threshold
+    unsigned long long lo = 0, hi = ~0ull;
     for (uint64_t i0 = tid & ~31ull; i0 < n; i0 += nth) {
         const uint64_t i = i0 + (threadIdx.x & 31);
         bool less = true;
@@ -175,6 +190,8 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(SplitArgs a) {
             const unsigned long long key = order_key(a.evec[i]);
             less = key < kpre || (key == kpre && (uint32_t)i < ipre);
             a.part[i] = less ? 0u : 1u;
+            if (less) lo = key > lo ? key : lo;
+            else if ((uint32_t)i != ipre) hi = key < hi ? key : hi;
         }
         const unsigned b = __ballot_sync(0xFFFFFFFFu, !less);
         if ((threadIdx.x & 31) == 0) a.bits[i0 >> 5] = b;
@@ -183,6 +200,18 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(SplitArgs a) {
         a.out[1] = a.k;
         a.out[2] = ipre;
         a.out[3] = 0;
+    }
+    if (a.gap >= 0) {
+        for (int o = 16; o; o >>= 1) {
+            const unsigned long long l = __shfl_xor_sync(0xFFFFFFFFu, lo, o), h = __shfl_xor_sync(0xFFFFFFFFu, hi, o);
+            lo = l > lo ? l : lo;
+            hi = h < hi ? h : hi;
+        }
+        if ((threadIdx.x & 31) == 0) {
+            atomicMax(a.out + 4, lo);
+            atomicMin(a.out + 5, hi);
+        }
+        if (tid == 0) a.out[6] = kpre;
     }
 }
 
@@ -283,6 +312,13 @@ __global__ void __launch_bounds__(kSplitThreads) k_split_sweep(SplitArgs a) {
             }
         }
         a.out[0] = (unsigned long long)(best / 2);
+        if (a.gap >= 0) {
+            // below the threshold: who is in part 0; behind it, too, where the
+            // threshold's vertex is the sweep's
+            const double t = key_value(a.out[6]);
+            a.out[7] = (a.k > 0 && t - key_value(a.out[4]) <= a.gap) ||
+                       (a.sweep && a.k + 1 < a.n && key_value(a.out[5]) - t <= a.gap);
+        }
     }
 }
 
@@ -317,8 +353,9 @@ static int launch_split(cudaStream_t s, int num_sms, uint32_t grid, SplitArgs &a
 }
 
 int split_level(Context &C, const Level &L, const double *evec, int perc_imbalance, uint32_t *part,
-                uint64_t *edgecut, uint32_t *n_part0) {
+                uint64_t *edgecut, uint32_t *n_part0, bool *close) {
     const uint32_t n = L.n;
+    if (close) *close = false;
     if (n == 0) { *edgecut = 0; if (n_part0) *n_part0 = 0; return SGP_B200_OK; }
     if (perc_imbalance != 0) {
         set_error("perc_imbalance_allowed must be 0 (the value sgpar.cpp passes); got %d", perc_imbalance);
@@ -338,7 +375,8 @@ int split_level(Context &C, const Level &L, const double *evec, int perc_imbalan
     SGPB_TRY(dalloc_t(C, &a.cand, 2 * kSelSmall));
     SGPB_TRY(dalloc_t(C, &a.bits, bit_words(n)));
     SGPB_TRY(dalloc_t(C, &a.longs, n));
-    SGPB_TRY(dalloc_t(C, &a.out, 4));
+    SGPB_TRY(dalloc_t(C, &a.out, kSplitOutWords));
+    a.gap = close ? kTieGap / sqrt((double)n) : -1.0;
     int per_sm = 0;
     SGPB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)k_split, kSplitThreads, 0));
     if (per_sm < 1) { set_error("split kernel does not fit"); return SGP_B200_ERR_DEVICE; }
@@ -349,8 +387,9 @@ int split_level(Context &C, const Level &L, const double *evec, int perc_imbalan
     if (grid < 1) grid = 1;
     SGPB_TRY(launch_split(C.stream, C.num_sms, grid, a));
     C.kernel_launches += 3;
-    uint64_t out[3];
-    SGPB_TRY(read_u64(C, (const uint64_t *)a.out, out, 3));
+    uint64_t out[kSplitOutWords];
+    SGPB_TRY(read_u64(C, (const uint64_t *)a.out, out, close ? kSplitOutWords : 3));
+    if (close) *close = out[7] != 0;
     *edgecut = out[0];
     if (n_part0) *n_part0 = (uint32_t)out[1];
     return SGP_B200_OK;
@@ -776,6 +815,7 @@ extern "C" int sgp_b200_split_noalloc(void *stream, uint32_t n, const uint32_t *
     const uint32_t imbl = n - imbr;
     a.k = imbl < n ? imbl : n - 1;
     a.sweep = imbr > imbl ? 1u : 0u;
+    a.gap = -1.0;
     a.longs = reinterpret_cast<uint32_t *>(d->scratch);
     a.bits = reinterpret_cast<uint32_t *>(d->scratch + kNoAllocBitsOff);
     a.cand = reinterpret_cast<unsigned long long *>(d->scratch + kNoAllocCandOff);

@@ -1,0 +1,104 @@
+"""Partitions do not depend on the order in which the power iteration adds up.
+
+Row slices and the rows form of the small levels add in another order than the
+plain kernels (SGPB_PI_SLICES=0), so their vectors differ by rounding.  A
+partition is certified against that (eigen.cu pi_plain, internal.h) and
+repeated in the plain order where the certificate fails: the median among
+values that are equal in exact arithmetic (leaves of one aggregate), an
+iteration that stops within rounding of the tolerance, an iterate that
+cancels.  Bit for bit against the plain order."""
+import numpy as np
+import pytest
+
+from ipdps_2021_graph_coarsening_b200 import graphs as G
+from tests.test_gpu_parity import dev_u32
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def of_edges(n, u, v):
+    k = np.unique(np.concatenate([u * n + v, v * n + u]))
+    rp = np.zeros(n + 1, np.uint32)
+    rp[1:] = np.cumsum(np.bincount(k // n, minlength=n))
+    return G.CSR(rp, (k % n).astype(np.uint32))
+
+
+def leafy(core, leaves, seed):
+    """An Erdos-Renyi core with leaves, most of them on its first vertices."""
+    c = G.erdos_renyi(core, 6.0, seed=seed)
+    rng = np.random.default_rng(seed)
+    u = np.repeat(np.arange(c.n), np.diff(c.row_ptr.astype(np.int64)))
+    hub = (c.n * rng.random(leaves) ** 4).astype(np.int64)
+    return of_edges(c.n + leaves, np.concatenate([u, hub]),
+                    np.concatenate([c.col.astype(np.int64), c.n + np.arange(leaves)]))
+
+
+# graphs whose parts (leafy, R-MAT 15), iteration counts and cut (R-MAT 14)
+# differ between the two orders
+GRAPHS = [(lambda s: leafy(8000, 12000, s), (7, 17, 27, 53)), (lambda s: leafy(3000, 30000, s), (13, 17, 51)),
+          (lambda s: G.rmat(15, 4, seed=s), (30, 51)), (lambda s: G.rmat(14, seed=s), (14, 41)),
+          (lambda s: G.rmat(13, seed=s), (42,))]
+
+
+def both(monkeypatch, call):
+    monkeypatch.delenv("SGPB_PI_SLICES", raising=False)
+    a = call()
+    monkeypatch.setenv("SGPB_PI_SLICES", "0")
+    return a, call()
+
+
+def same(a, b):
+    assert np.array_equal(a.part, b.part)
+    assert (a.edgecut, a.part0_size, a.level_iters, a.rng_state) == (b.edgecut, b.part0_size, b.level_iters, b.rng_state)
+
+
+@pytest.mark.parametrize("make,seed", [(f, s) for f, seeds in GRAPHS for s in seeds])
+def test_partitions_are_the_plain_order_s(partitioner, monkeypatch, make, seed):
+    g = make(seed)
+    same(*both(monkeypatch, lambda: partitioner.partition(g, rng_state=1000 + seed)))
+
+
+def test_batch_and_4way_are_the_plain_order_s(partitioner, monkeypatch):
+    gs = [make(s) for make, seeds in GRAPHS[:2] for s in seeds]
+    for a, b in zip(*both(monkeypatch, lambda: partitioner.partition_batch(gs, rng_state=1007))):
+        same(a, b)
+    # two vertices joined by an edge: r = 0, and what is left is rounding
+    tri = of_edges(3, np.array([0, 0, 1]), np.array([1, 2, 2]))
+    for g in (tri, gs[0]):
+        for seed in range(70, 80):
+            a, b = both(monkeypatch, lambda: partitioner.partition_4way(g, rng_state=seed))
+            assert np.array_equal(a[0], b[0]) and a[1:] == b[1:]
+
+
+@pytest.mark.parametrize("n", [700, 20000])   # one block's rows form, row slices
+def test_a_stop_within_rounding_of_the_tolerance(partitioner, monkeypatch, n):
+    g = G.erdos_renyi(n, 8.0, seed=3)
+    rp, col = dev_u32(g.row_ptr), dev_u32(g.col)
+    x = torch.from_numpy(np.random.default_rng(1).random(g.n)).cuda()
+
+    def run(tol):
+        y, iters, lam, _ = partitioner.power_iter(rp, col, None, x, tol=tol, residual=False)
+        return y.cpu().numpy(), iters
+
+    # the tolerance at which the plain order takes one iteration more
+    monkeypatch.setenv("SGPB_PI_SLICES", "0")
+    k = run(1e-7)[1]
+    lo, hi = 1e-8, 1e-7   # more than k, at most k
+    assert run(lo)[1] > k
+    while hi - lo > 1e-17:
+        mid = 0.5 * (lo + hi)
+        if run(mid)[1] > k:
+            lo = mid
+        else:
+            hi = mid
+    for tol in (lo, hi, lo - 2e-16, hi + 2e-16):
+        (a, ia), (b, ib) = both(monkeypatch, lambda: run(tol))
+        assert ia == ib and np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [700, 20000])
+def test_tolerances_near_rounding_take_the_plain_order(partitioner, monkeypatch, n):
+    g = G.erdos_renyi(n, 8.0, seed=4)
+    for tol in (9e-12, 1e-14, 0.0):
+        same(*both(monkeypatch, lambda: partitioner.partition(g, tol=tol, iter_cap=400, rng_state=5)))
