@@ -81,6 +81,8 @@ struct SliceArgs {
     const uint32_t *sptr;         // [n+1] chunk slots of each row
     uint32_t nslots;
     double *spart;                // sums of chunks
+    uint32_t ncross;              // (direct) > 0: the chunks of a row are anywhere, its rows are added up ...
+    const uint32_t *cross;        // ... behind a second barrier: the rows with chunks, ascending
     double *y;                    // [P][n32] row sums of the panels
     const double *deg;            // [n] weighted degrees
     const uint32_t *inv;          // new id -> level vertex id (null: identity)
@@ -379,8 +381,9 @@ __device__ __forceinline__ void warp_units(const SliceArgs &a, uint32_t u, uint3
     k1 = wid + 1 == kSliceWarps ? ue : slice_lower_bound(a.cpre, u, ue, c0 + (c1 - c0) * (wid + 1) / kSliceWarps);
 }
 
-// FORM: the level's form; WB: bytes per weight (0: none).
-template <int FORM, int WB>
+// FORM: the level's form; WB: bytes per weight (0: none); CROSS: a row's chunks
+// are anywhere (ncross; as a branch it cost every other level 0.25 us an iteration).
+template <int FORM, int WB, bool CROSS>
 __global__ void __launch_bounds__(slice_threads(FORM, WB), 1) k_pi_slices(SliceArgs a) {
     constexpr int kSliceThreads = slice_threads(FORM, WB), kSliceWarps = kSliceThreads / 32;
     constexpr bool PANELS = FORM == kFormPanels, GLOBAL = FORM == kFormGlobal || FORM == kFormHub;
@@ -402,13 +405,14 @@ __global__ void __launch_bounds__(slice_threads(FORM, WB), 1) k_pi_slices(SliceA
     double *part0 = a.partials, *part1 = a.partials + 4 * (size_t)gridDim.x;
     if (COPY && threadIdx.x < kBanks) xs[kSlicePW + threadIdx.x] = 0.0;
     // units of this block: an equal share of the cost; the direct forms keep
-    // the units of a row (its chunks) in one block
+    // the units of a row (its chunks) in one block, unless a row is much longer
+    // than a block's share (ncross)
     const uint64_t call = a.cpre[a.nu];
     auto block_unit = [&](uint32_t b) -> uint32_t {
         if (b == 0) return 0u;
         if (b >= gridDim.x) return a.nu;
         uint32_t u = slice_lower_bound(a.cpre, 0, a.nu, call * b / gridDim.x);
-        if (!PANELS)
+        if (!PANELS && !CROSS)
             while (u < a.nu && u > 0 && a.unit[u].y == a.unit[u - 1].y) u++;
         return u;
     };
@@ -634,7 +638,16 @@ __global__ void __launch_bounds__(slice_threads(FORM, WB), 1) k_pi_slices(SliceA
                 else if (d.w != 0xFFFFFFFFu && lane == 0) a.spart[d.w] = s;
                 if (more) fetch(dn);
             });
-            if (a.nslots) {
+            if (CROSS) {
+                if (!bar.sync(&s_ok)) return;
+                for (uint32_t q = blockIdx.x * kSliceWarps + wid; q < a.ncross; q += gridDim.x * kSliceWarps) {
+                    const uint32_t i = a.cross[q];
+                    double acc = 0;
+                    for (uint32_t k = a.sptr[i] + lane; k < a.sptr[i + 1]; k += 32) acc += __ldcg(a.spart + k);
+                    acc = warp_sum(acc);
+                    if (lane == 0) fin(i, acc, own(i), a.deg[i]);
+                }
+            } else if (a.nslots) {
                 __syncthreads();   // the chunks of the block's rows are summed
                 for (uint32_t i = R0 + threadIdx.x; i < R1; i += kSliceThreads) {
                     const uint32_t b = a.sptr[i], e = a.sptr[i + 1];
@@ -719,7 +732,7 @@ __global__ void k_sl_lead(const uint32_t *rp, const uint32_t *inv, unsigned long
 
 struct SliceBuild {
     uint32_t n, n32, ng, P, epl, nitems;
-    int direct, expand;
+    int direct, expand, l2;
     const uint32_t *rp, *col;
     const void *w;
     const uint32_t *perm, *inv;          // null: identity
@@ -833,6 +846,11 @@ __global__ void __launch_bounds__(32 * kLayWarps) k_sl_row_counts(SliceBuild b) 
     }
 }
 
+__global__ void k_sl_chunked(uint32_t n, const uint32_t *sptr, uint8_t *flags) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) flags[i] = sptr[i + 1] > sptr[i];
+}
+
 // row lengths in the layout's numbering (one panel) and weighted degrees
 __global__ void k_sl_degrees(SliceBuild b) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -894,7 +912,10 @@ __global__ void __launch_bounds__(256) k_sl_groups(SliceBuild b) {
 // cost of a unit in the split over blocks and warps, in half steps: its steps,
 // a quarter more where every lane has a row of its own (short rows share banks
 // more often: R-MAT 22's level 1 122 -> 118 us), plus the price of two steps for
-// the record, the butterfly and the row's value
+// the record, the butterfly and the row's value.  Gathers from L2 (l2) cost by
+// their number too: rows of a few entries leave most places of a step empty, and
+// 512 rows of 2,000 entries among a million of five had 7 blocks to themselves
+// (66 -> 31 us; entries / 64 in place of / 16: 45)
 __global__ void __launch_bounds__(256) k_sl_units(SliceBuild b) {
     const unsigned lane = threadIdx.x & 31;
     const uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -919,10 +940,12 @@ __global__ void __launch_bounds__(256) k_sl_units(SliceBuild b) {
     if (t == (uint64_t)b.P * b.ng - 1 && lane == 31) b.pan_u[b.P] = b.unb[t] + us;
     b.roff[(size_t)p * b.n32 + i] = __shfl_sync(0xFFFFFFFFu, off, lane & ~((32u >> r.lg) - 1u));
     b.rst[(size_t)p * b.n32 + i] = r.steps | (r.lg << 24);
+    uint32_t entries = r.len;   // of the unit
+    for (uint32_t o = 1; o < (32u >> r.lg); o <<= 1) entries += __shfl_xor_sync(0xFFFFFFFFu, entries, o);
     if (!nu) return;
     if (r.chunks <= 1) {
         b.unit[u0] = make_uint4(off, i, r.steps | (r.lg << 16), 0xFFFFFFFFu);
-        b.ucost[u0] = 2 * r.steps + (r.lg == 0 ? r.steps / 2 : 0) + 4;
+        b.ucost[u0] = 2 * r.steps + (b.l2 ? entries / 16 : r.lg == 0 ? r.steps / 2 : 0) + 4;
         return;
     }
     uint32_t slot = b.sptr[i];
@@ -934,7 +957,8 @@ __global__ void __launch_bounds__(256) k_sl_units(SliceBuild b) {
     for (uint32_t k = 0; k < r.chunks; k++) {
         const uint32_t st = k + 1 < r.chunks ? full : r.steps - k * full;
         b.unit[u0 + k] = make_uint4(off + k * full, i, st | (5u << 16), slot + k);
-        b.ucost[u0 + k] = 2 * st + 4;
+        const uint32_t left = r.len - k * 32 * b.epl;
+        b.ucost[u0 + k] = 2 * st + (b.l2 ? (left < 32 * b.epl ? left : 32 * b.epl) / 16 : 0) + 4;
     }
 }
 
@@ -1141,6 +1165,14 @@ constexpr uint64_t kMaxCopies = 4096;
 // SM
 constexpr uint64_t kHubTail = 1ull << 20;
 
+// A row in one block takes its entries' time there: a row this much longer than
+// a block's share (gathers from L2 / from shared memory) costs more than the
+// second barrier, about 3 us.  A star of 100,000 vertices 39 -> 9 us an iteration
+// (the main kernel 33), of 30,000 and 60,000 random pairs 18 -> 9.2 (12), 4 hubs
+// among 1,000,000 vertices of six entries 142 -> 38 (105); rows of 7,500 in the
+// hub form are quicker in one block (8.7 against 9.6).
+constexpr uint64_t kLongRowGlobal = 4096, kLongRowShared = 16384;
+
 // The form of a level.  skew: its longest row is at least four times the mean;
 // tail: its entries beyond the leading kSlicePW vertices in degree order.
 // Mesh level of 57,210 vertices, 4.1 entries per row and panel: panels 12.6 us
@@ -1159,15 +1191,20 @@ bool power_iter_slices_ok(const Level &L, const PowerIterOpts &o) {
     return L.wbytes == 0 || L.wbytes == 4 || L.wbytes == 8;
 }
 
-template <int FORM>
+template <int FORM, bool CROSS>
 static const void *slice_kernel(int wb) {
     switch (wb) {
-        case 0: return (const void *)k_pi_slices<FORM, 0>;
-        case 1: return (const void *)k_pi_slices<FORM, 1>;
-        case 2: return (const void *)k_pi_slices<FORM, 2>;
-        case 4: return (const void *)k_pi_slices<FORM, 4>;
-        default: return (const void *)k_pi_slices<FORM, 8>;
+        case 0: return (const void *)k_pi_slices<FORM, 0, CROSS>;
+        case 1: return (const void *)k_pi_slices<FORM, 1, CROSS>;
+        case 2: return (const void *)k_pi_slices<FORM, 2, CROSS>;
+        case 4: return (const void *)k_pi_slices<FORM, 4, CROSS>;
+        default: return (const void *)k_pi_slices<FORM, 8, CROSS>;
     }
+}
+
+template <int FORM>
+static const void *direct_kernel(int wb, bool cross) {
+    return cross ? slice_kernel<FORM, true>(wb) : slice_kernel<FORM, false>(wb);
 }
 
 template <typename WI>
@@ -1267,6 +1304,7 @@ static int slices_run(Context &C, const Level &L, const double *x_in, const uint
     const SliceForm form = slice_form(n, L.m, skew, tail);
     if (form == kFormGlobal) b.perm = b.inv = nullptr;   // its gathers keep the level's locality
     const bool wide = form == kFormGlobal || form == kFormHub;   // 32-bit destinations, places by rank
+    b.l2 = form == kFormGlobal;
     b.direct = form != kFormPanels;
     b.P = form == kFormPanels ? cdiv(n, kSlicePW) : 1u;
     // (one lane writes an entry's copies: at most kMaxCopies)
@@ -1369,6 +1407,18 @@ static int slices_run(Context &C, const Level &L, const double *x_in, const uint
     a.col = b.ocol; a.w = b.ow; a.sptr = sptr; a.nslots = nslots; a.deg = deg; a.inv = b.inv;
     a.x_in = x_in; a.vcmap = vcmap; a.out = x_out;
     SGPB_TRY(dalloc_t(C, &a.spart, (size_t)nslots + 1));
+    if (b.direct && nslots && maxlen > me / C.num_sms + (b.l2 ? kLongRowGlobal : kLongRowShared)) {
+        uint8_t *flags;
+        uint32_t *list, *cnt;
+        SGPB_TRY(dalloc_t(C, &flags, n));
+        SGPB_TRY(dalloc_t(C, &list, (size_t)n + 1));
+        SGPB_TRY(dalloc_t(C, &cnt, 1));
+        k_sl_chunked<<<cdiv(n, 256), 256, 0, C.stream>>>(n, sptr, flags);
+        C.kernel_launches++;
+        SGPB_TRY(compact_flags(C, flags, n, list, cnt));
+        SGPB_TRY(read_u32(C, cnt, &a.ncross));
+        a.cross = list;
+    }
     SGPB_TRY(dalloc_t(C, &a.va, b.n32));
     SGPB_TRY(dalloc_t(C, &a.vb, b.n32));
     SGPB_CUDA(cudaMemsetAsync(a.va + (n & ~1u), 0, sizeof(double) * (b.n32 - (n & ~1u)), C.stream));
@@ -1394,10 +1444,10 @@ static int slices_run(Context &C, const Level &L, const double *x_in, const uint
     if (C.grid_cap && grid > C.grid_cap) grid = C.grid_cap;
     if (grid < 1) grid = 1;
     SGPB_TRY(dalloc_t(C, &a.partials, (size_t)8 * grid));
-    const void *k = form == kFormShared   ? slice_kernel<kFormShared>(wb)
-                    : form == kFormGlobal ? slice_kernel<kFormGlobal>(wb)
-                    : form == kFormHub    ? slice_kernel<kFormHub>(wb)
-                                          : slice_kernel<kFormPanels>(wb);
+    const void *k = form == kFormShared   ? direct_kernel<kFormShared>(wb, a.ncross != 0)
+                    : form == kFormGlobal ? direct_kernel<kFormGlobal>(wb, a.ncross != 0)
+                    : form == kFormHub    ? direct_kernel<kFormHub>(wb, a.ncross != 0)
+                                          : slice_kernel<kFormPanels, false>(wb);
     const size_t dyn = form == kFormGlobal ? 0 : kSliceSmem;
     if (dyn) SGPB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSliceSmem));
     cudaEvent_t ev[2];

@@ -6,6 +6,8 @@ items, unit, repeated, 8-, 16-, 32- and 64-bit weights, rows without entries.
 Against the oracle after a fixed number of iterations: each iteration rounds
 the FP64 iterate to about 1e-16 per operation, so 40 of them stay well within
 1e-11 of its norm."""
+import time
+
 import numpy as np
 import pytest
 
@@ -185,3 +187,44 @@ def test_small_level_dense(partitioner):
     rp, col = csr(90, rng.integers(0, 90, 9000), rng.integers(0, 90, 9000))
     check(partitioner, rp, col, weights(rp, col, 1000))
     check(partitioner, rp, col, weights(rp, col, (1 << 33) + 1), wide=True)
+
+
+def star(n, hubs, extra):
+    """Every vertex joined to one of the first few, and random pairs."""
+    rng = np.random.default_rng(n)
+    i = np.arange(n)
+    return csr(n, np.concatenate([i % hubs, rng.integers(0, n, extra)]), np.concatenate([i, rng.integers(0, n, extra)]))
+
+
+# the iterate in shared memory, its leading part there, and gathers from L2 in
+# the level's and (a skewed level wider than its panels pay for) its own order;
+# one row, or several, far above a block's share of the entries
+@pytest.mark.parametrize("n,hubs,extra", [(25001, 1, 0), (25001, 1, 50000), (40000, 1, 80000), (100001, 1, 0),
+                                          (100001, 3, 100000), (200001, 2, 1600000)])
+@pytest.mark.parametrize("top", [0, 200, 60000, 1 << 31])
+def test_rows_above_a_block_s_share(partitioner, n, hubs, extra, top):
+    rp, col = star(n, hubs, extra)
+    check(partitioner, rp, col, weights(rp, col, top) if top else None)
+    if top == 200:
+        check(partitioner, rp, col, weights(rp, col, (1 << 33) + 5), wide=True)
+
+
+@pytest.mark.parametrize("n,hubs,extra", [(100001, 1, 0), (100001, 4, 100000), (300001, 4, 600000)])
+def test_long_rows_are_not_slower(partitioner, monkeypatch, n, hubs, extra):
+    """300 iterations with few long rows take no longer than on the main kernel
+    (1.1 to 1.8 times as long where one block had the whole of such a row)."""
+    rp, col = star(n, hubs, extra)
+    rp, col = dev(rp), dev(col)
+    x = torch.from_numpy(np.random.default_rng(1).random(n)).cuda()
+
+    def best():
+        t = []
+        for _ in range(6):
+            t0 = time.perf_counter()
+            partitioner.power_iter(rp, col, None, x, tol=-1.0, iter_cap=300, residual=False)
+            t.append(time.perf_counter() - t0)
+        return min(t)
+
+    fast = best()
+    monkeypatch.setenv("SGPB_PI_SLICES", "0")
+    assert fast <= best()
