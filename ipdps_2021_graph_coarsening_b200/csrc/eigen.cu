@@ -2805,11 +2805,21 @@ static int autotune_level(Context &C, const Level &L, const PIArgs &a0, bool mix
     return SGP_B200_OK;
 }
 
-// Iterations a level with o.probe takes before its row slices are laid out,
-// and the entries below which it is laid out at once.  R-MAT 22's input level
-// stops after two.
+// Iterations a level with o.probe takes before its row slices are laid out, and
+// the entries below which it is laid out at once (R-MAT 22's input level stops
+// after two); calls of at most as many iterations do without the layout, which
+// costs as much as a few of them.
 constexpr uint64_t kProbeIters = 4;
 constexpr uint64_t kProbeMinM = 1ull << 20;
+
+bool pi_plain(const PowerIterOpts &o) {
+    if (o.plain || o.mixed || o.normlap || (o.tol >= 0 && o.tol < kPlainTol)) return true;
+    if (o.iter_cap && o.iter_cap <= kProbeIters) return true;
+    if (const char *e = getenv("SGPB_PI_MODE"))
+        if (*e) return true;
+    const char *e = getenv("SGPB_PI_SLICES");
+    return e && atoi(e) == 0;
+}
 
 int power_iter_level(Context &C, const Level &Lin, const double *x_in, const uint32_t *vcmap, double *x_out,
                      const PowerIterOpts &o, PowerIterResult *res, int want_residual) {
@@ -3011,14 +3021,6 @@ int level_residual(Context &C, const Level &L, const double *x, int normlap, Pow
     const double scale = normlap ? 2.0 : (res->gb > 0 ? res->gb : 1);   // bound on the spectrum
     res->resid = sqrt(r2 / (x2 > 0 ? x2 : 1)) / scale;
     return SGP_B200_OK;
-}
-
-bool pi_plain(const PowerIterOpts &o) {
-    if (o.plain || o.mixed || o.normlap || (o.tol >= 0 && o.tol < kPlainTol)) return true;
-    if (const char *e = getenv("SGPB_PI_MODE"))
-        if (*e) return true;
-    const char *e = getenv("SGPB_PI_SLICES");
-    return e && atoi(e) == 0;
 }
 
 bool power_iter_small_ok(const Level &L, const PowerIterOpts &o) {

@@ -204,7 +204,7 @@ constexpr double kStopMargin = 1e-15;
 // products, so that the number of iterations is the rounding's
 constexpr double kPlainTol = 1e-11;
 // whether levels run in the plain order: asked for, a tolerance below
-// kPlainTol, mixed precision (whose FP32 differences amplify any other
+// kPlainTol, a cap of very few iterations, mixed precision (whose FP32 differences amplify any other
 // rounding), the normalized walk (no deflation in its loop), a forced kernel
 // (SGPB_PI_MODE), or SGPB_PI_SLICES=0
 bool pi_plain(const PowerIterOpts &o);

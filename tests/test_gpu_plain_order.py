@@ -37,6 +37,7 @@ def leafy(core, leaves, seed):
 # graphs whose parts (leafy, R-MAT 15), iteration counts and cut (R-MAT 14)
 # differ between the two orders
 GRAPHS = [(lambda s: leafy(8000, 12000, s), (7, 17, 27, 53)), (lambda s: leafy(3000, 30000, s), (13, 17, 51)),
+          (lambda s: leafy(8000, 6000, s), (15, 27, 31, 120)),
           (lambda s: G.rmat(15, 4, seed=s), (30, 51)), (lambda s: G.rmat(14, seed=s), (14, 41)),
           (lambda s: G.rmat(13, seed=s), (42,))]
 
@@ -102,3 +103,12 @@ def test_tolerances_near_rounding_take_the_plain_order(partitioner, monkeypatch,
     g = G.erdos_renyi(n, 8.0, seed=4)
     for tol in (9e-12, 1e-14, 0.0):
         same(*both(monkeypatch, lambda: partitioner.partition(g, tol=tol, iter_cap=400, rng_state=5)))
+
+
+@pytest.mark.parametrize("n", [700, 20000])
+def test_a_few_iterations_do_without_the_layout(partitioner, monkeypatch, n):
+    g = G.erdos_renyi(n, 8.0, seed=5)
+    rp, col = dev_u32(g.row_ptr), dev_u32(g.col)
+    x = torch.from_numpy(np.random.default_rng(2).random(g.n)).cuda()
+    a, b = both(monkeypatch, lambda: partitioner.power_iter(rp, col, None, x, iter_cap=4, residual=False))
+    assert a[1] == b[1] == 4 and torch.equal(a[0], b[0])
