@@ -50,10 +50,11 @@ __global__ void k_sum_u32(const uint32_t *w, uint64_t m, unsigned long long *out
 }
 
 __global__ void k_check_csr(uint32_t n, uint64_t m, const uint32_t *rp, const uint32_t *col, uint32_t *bad) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && rp[i + 1] < rp[i]) atomicOr(bad, 1u);
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t u = i; u < n; u += step)
+        if (rp[u + 1] < rp[u]) atomicOr(bad, 1u);
     if (i == 0 && (rp[0] != 0 || rp[n] != m)) atomicOr(bad, 2u);
-    for (uint64_t j = i; j < m; j += (uint64_t)gridDim.x * blockDim.x)
+    for (uint64_t j = i; j < m; j += step)
         if (col[j] >= n) { atomicOr(bad, 4u); break; }
 }
 
