@@ -49,10 +49,17 @@ __global__ void k_sum_u32(const uint32_t *w, uint64_t m, unsigned long long *out
     if ((threadIdx.x & 31) == 0 && s) atomicAdd(out, (unsigned long long)s);
 }
 
+// bad[0]: what is wrong; bad[1]: vertices of one entry
 __global__ void k_check_csr(uint32_t n, uint64_t m, const uint32_t *rp, const uint32_t *col, uint32_t *bad) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t u = i; u < n; u += step)
-        if (rp[u + 1] < rp[u]) atomicOr(bad, 1u);
+    uint32_t leaves = 0;
+    for (uint64_t u = i; u < n; u += step) {
+        const uint32_t b = rp[u], e = rp[u + 1];
+        if (e < b) atomicOr(bad, 1u);
+        leaves += e - b == 1;
+    }
+    leaves = warp_sum(leaves);
+    if ((threadIdx.x & 31) == 0 && leaves) atomicAdd(bad + 1, leaves);
     if (i == 0 && (rp[0] != 0 || rp[n] != m)) atomicOr(bad, 2u);
     for (uint64_t j = i; j < m; j += step)
         if (col[j] >= n) { atomicOr(bad, 4u); break; }
@@ -93,19 +100,20 @@ static int stage_input(Context &C, const sgp_b200_graph_t *g, Level *L0) {
         }
     }
     uint32_t *bad;
-    SGPB_TRY(dalloc_t(C, &bad, 1));
-    SGPB_TRY(dzero(C, bad, 4));
+    SGPB_TRY(dalloc_t(C, &bad, 2));
+    SGPB_TRY(dzero(C, bad, 8));
     uint32_t blocks = cdiv(g->n + 1, 256);
     if (blocks > (uint32_t)C.num_sms * 8) blocks = C.num_sms * 8;
     k_check_csr<<<blocks, 256, 0, C.stream>>>(g->n, g->m, L0->rp, L0->col, bad);
     C.kernel_launches++;
-    uint32_t hb = 0;
-    SGPB_TRY(read_u32(C, bad, &hb));
-    if (hb) {
+    uint32_t hb[2] = {0, 0};
+    SGPB_TRY(read_u32(C, bad, hb, 2));
+    if (hb[0]) {
         set_error("malformed CSR (code %u: 1 = decreasing offsets, 2 = row_ptr[0] != 0 or row_ptr[n] != m, "
-                  "4 = destination >= n)", hb);
+                  "4 = destination >= n)", hb[0]);
         return SGP_B200_ERR_INVALID;
     }
+    L0->leaves = hb[1];
     return SGP_B200_OK;
 }
 
@@ -380,6 +388,10 @@ static int partition_begin(Context &C, const Level &L0, const sgp_b200_options_t
     S->po.iter_cap = opt->iter_cap;
     S->po.mixed = opt->mixed;
     S->po.normlap = opt->refine_alg == 1;
+    // leaves of one aggregate are equal (internal.h): where most vertices are
+    // leaves the median falls among such most of the time, and the fast order,
+    // which takes about half the plain one's time, is not worth trying
+    S->po.plain = 2ull * L0.leaves > L0.n;
     // the cluster kernel's share of the levels: up to 2^23 cost units in a
     // batch (many levels at once); the levels' own rule in a single partition
     const uint32_t lg = opt->cluster_max_log2 ? (opt->cluster_max_log2 < 40 ? opt->cluster_max_log2 : 40u)

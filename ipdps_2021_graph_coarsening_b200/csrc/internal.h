@@ -108,6 +108,7 @@ struct Level {
     uint32_t *vtx_w = nullptr;   // vertex weights; null: every vertex weighs 1 (the input level)
     uint32_t *wmax = nullptr;    // device word: the largest 32-bit weight (tiered builds), null: unknown
     uint32_t max_deg = 0;
+    uint32_t leaves = 0;         // vertices of one entry (input levels; 0 where not counted)
     uint32_t seed_hi = 0, seed_lo = 0;
     int hec_rounds = 0;
     uint64_t pi_iters = 0;
