@@ -913,9 +913,10 @@ __global__ void __launch_bounds__(256) k_sl_groups(SliceBuild b) {
 // a quarter more where every lane has a row of its own (short rows share banks
 // more often: R-MAT 22's level 1 122 -> 118 us), plus the price of two steps for
 // the record, the butterfly and the row's value.  Gathers from L2 (l2) cost by
-// their number too: rows of a few entries leave most places of a step empty, and
-// 512 rows of 2,000 entries among a million of five had 7 blocks to themselves
-// (66 -> 31 us; entries / 64 in place of / 16: 45)
+// their number too, and a unit the price of four steps: rows of a few entries
+// leave most places of a step empty, and 512 rows of 2,000 entries among a million
+// of six had 7 blocks to themselves (79 -> 51 us; with a unit at two steps 36, but
+// the weighted Chung-Lu input of 262,147 vertices 47 in place of 39.5 -> 38.4)
 __global__ void __launch_bounds__(256) k_sl_units(SliceBuild b) {
     const unsigned lane = threadIdx.x & 31;
     const uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -945,7 +946,7 @@ __global__ void __launch_bounds__(256) k_sl_units(SliceBuild b) {
     if (!nu) return;
     if (r.chunks <= 1) {
         b.unit[u0] = make_uint4(off, i, r.steps | (r.lg << 16), 0xFFFFFFFFu);
-        b.ucost[u0] = 2 * r.steps + (b.l2 ? entries / 16 : r.lg == 0 ? r.steps / 2 : 0) + 4;
+        b.ucost[u0] = b.l2 ? 4 * r.steps + entries / 16 + 16 : 2 * r.steps + (r.lg == 0 ? r.steps / 2 : 0) + 4;
         return;
     }
     uint32_t slot = b.sptr[i];
@@ -958,7 +959,7 @@ __global__ void __launch_bounds__(256) k_sl_units(SliceBuild b) {
         const uint32_t st = k + 1 < r.chunks ? full : r.steps - k * full;
         b.unit[u0 + k] = make_uint4(off + k * full, i, st | (5u << 16), slot + k);
         const uint32_t left = r.len - k * 32 * b.epl;
-        b.ucost[u0 + k] = 2 * st + (b.l2 ? (left < 32 * b.epl ? left : 32 * b.epl) / 16 : 0) + 4;
+        b.ucost[u0 + k] = b.l2 ? 4 * st + (left < 32 * b.epl ? left : 32 * b.epl) / 16 + 16 : 2 * st + 4;
     }
 }
 
