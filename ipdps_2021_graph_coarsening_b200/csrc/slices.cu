@@ -67,7 +67,7 @@ __host__ __device__ constexpr int slice_threads(int form, int wb) {
 constexpr uint32_t kSliceItem = 2048;       // entries of a row that one warp lays out
 constexpr uint32_t kSliceMaxPanels = 32;    // a lane holds a panel's bounds in the layout kernels
 constexpr int kSumK = 3;                    // sum r, sum r^2, sum u r
-constexpr uint32_t kSpinLimit = 1u << 28;   // polls of a grid barrier before giving up
+constexpr uint32_t kSpinLimit = 1u << 23;   // polls of a grid barrier before giving up, about 6 s
 
 
 struct SliceArgs {
@@ -91,8 +91,9 @@ struct SliceArgs {
     double *va, *vb;              // n32 doubles each, zero behind n
     double *out;
     double *partials;             // [2][grid][4]
-    uint32_t *bar;                // grid barrier counter, 0 at launch
-    uint32_t *err;
+    uint32_t *bar;                // grid barrier counter and err, 0 at launch; 8-byte aligned
+    uint32_t *err;                // set by a block that gave up waiting; the others leave at their next barrier
+    uint32_t spin;                // polls of a grid barrier before giving up
     double tol;
     uint64_t iter_max;
     double *res;                  // [0] niter [1] dot [2] gb [3] lambda [4] capped [5] barrier gave up
@@ -104,11 +105,12 @@ struct SliceArgs {
 
 // ------------------------------------------------------------- barrier --
 // Grid barrier of a cooperative launch: arrivals are counted in one word that
-// only grows, thread 0 polls it with a limit.  Returns false when the limit
-// ran out here or in another block (the kernel then returns).
+// only grows, thread 0 polls it with a limit.  Returns false, and the kernel
+// then returns, when the limit ran out here (err is set), or err was set before
+// or while this block waited (err is the word behind the counter, one load).
 struct GridBar {
-    uint32_t *ctr, *err;
-    uint32_t target;
+    uint32_t *ctr;
+    uint32_t target, limit;
     // by warp 0 alone, after a block barrier behind the other warps' stores
     __device__ __forceinline__ void arrive() {
         target += gridDim.x;
@@ -120,12 +122,14 @@ struct GridBar {
     // by every thread; target is warp 0's
     __device__ __forceinline__ bool wait(uint32_t *s_ok) {
         if (threadIdx.x == 0) {
-            uint32_t v = 0, k = 0;
+            unsigned long long both;
+            uint32_t k = 0;
             do {
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ctr) : "memory");
-            } while ((int32_t)(v - target) < 0 && ++k < kSpinLimit);
-            if ((int32_t)(v - target) < 0) atomicExch(err, 1u);
-            *s_ok = (int32_t)(v - target) >= 0 ? 1u : 0u;
+                asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(both) : "l"(ctr) : "memory");
+            } while ((int32_t)((uint32_t)both - target) < 0 && !(both >> 32) && ++k < limit);
+            const bool ok = (int32_t)((uint32_t)both - target) >= 0 && !(both >> 32) && limit;
+            if (!ok) atomicExch(ctr + 1, 1u);
+            *s_ok = ok ? 1u : 0u;
         }
         __syncthreads();
         return *s_ok != 0;
@@ -364,9 +368,11 @@ struct PanelCopy {
             bulk_load((char *)xs + b, (const char *)src + b, bytes - b < per ? bytes - b : per, bar);
         }
     }
-    // by every thread; false when the wait limit ran out
+    // by every thread; false when the wait limit ran out (the copy is waited
+    // for once more, so that the block does not leave under it)
     __device__ __forceinline__ bool wait() {
         const bool ok = mbar_wait(bar, phase);
+        if (!ok) mbar_wait(bar, phase);
         phase ^= 1;
         return ok;
     }
@@ -398,7 +404,7 @@ __global__ void __launch_bounds__(slice_threads(FORM, WB), 1) k_pi_slices(SliceA
     const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t gtid = blockIdx.x * kSliceThreads + threadIdx.x, gthr = gridDim.x * kSliceThreads;
     __shared__ __align__(8) uint64_t s_mbar;
-    GridBar bar{a.bar, a.err, 0};
+    GridBar bar{a.bar, 0, a.spin};
     PanelCopy panel{&s_mbar, 0};
     if (threadIdx.x == 0) s_margin = 1e300;
     if (COPY) panel.init();   // seen by the block behind the start vector's barriers
@@ -1434,6 +1440,9 @@ static int slices_run(Context &C, const Level &L, const double *x_in, const uint
     SGPB_TRY(dzero(C, a.bar, 8));
     SGPB_TRY(dzero(C, res_d, 64));
     a.err = a.bar + 1;
+    a.spin = kSpinLimit;
+    if (const char *e = getenv("SGPB_PI_SPIN"))   // another limit (0: the first wait gives up)
+        if (*e) a.spin = (uint32_t)strtoul(e, nullptr, 10);
     a.res = res_d;
     a.tol = o.tol;
     a.iter_max = iter_max;

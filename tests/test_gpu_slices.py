@@ -228,3 +228,16 @@ def test_long_rows_are_not_slower(partitioner, monkeypatch, n, hubs, extra):
     fast = best()
     monkeypatch.setenv("SGPB_PI_SLICES", "0")
     assert fast <= best()
+
+
+@pytest.mark.parametrize("n,m", [(9000, 120000), (40000, 200000), (77000, 200000), (51201, 6000000)])
+def test_a_barrier_that_gives_up(partitioner, monkeypatch, n, m):
+    """The grid barrier's limit runs out in every form: an error, and the
+    context goes on."""
+    rp, col = skewed(n, m, 4)
+    monkeypatch.setenv("SGPB_PI_SPIN", "0")
+    x = torch.zeros(n, dtype=torch.float64, device="cuda")
+    with pytest.raises(RuntimeError, match="grid barrier did not complete"):
+        partitioner.power_iter(dev(rp), dev(col), None, x, tol=-1.0, iter_cap=CAP)
+    monkeypatch.delenv("SGPB_PI_SPIN")
+    check(partitioner, rp, col)
