@@ -657,9 +657,11 @@ static bool is_pinned(const void *p) {
 
 static bool is_pageable(const void *p) {
     cudaPointerAttributes at;
-    const bool plain = cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
-    cudaGetLastError();
-    return plain;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();   // its own error alone: one of an earlier launch stays to be found
+        return false;
+    }
+    return at.type == cudaMemoryTypeUnregistered;
 }
 
 // The whole text into `dtext` (capacity >= len): pinned host memory and device
@@ -701,8 +703,12 @@ static int upload_text(Context &C, MtxSource &src, uint8_t *dtext) {
 // destinations) 16.3 -> 7.9 ms, of R-MAT 19 9.2 -> 5.4, R-MAT 18 4.7 -> 4.0.
 int upload_host(Context &C, void *dst, const void *src, size_t bytes) {
     const size_t chunk = stage_slot(bytes, kUploadSlotBytes);
-    if (bytes < kUploadMin || !is_pageable(src) || ensure_stage(C, chunk) != SGP_B200_OK) {
+    bool ring = bytes >= kUploadMin && is_pageable(src);
+    if (ring && ensure_stage(C, chunk) != SGP_B200_OK) {
         cudaGetLastError();   // no pinned ring to be had
+        ring = false;
+    }
+    if (!ring) {
         SGPB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, C.stream));
         return SGP_B200_OK;
     }
