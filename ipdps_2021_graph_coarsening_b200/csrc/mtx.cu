@@ -548,7 +548,13 @@ class HostPool {
     HostPool() {
         const unsigned hw = std::thread::hardware_concurrency();
         const int w = hw > 8 ? 8 : (hw ? (int)hw : 1);
-        for (int i = 1; i < w; i++) th_.emplace_back([this] { loop(); });
+        // as many as there are to be had: an exception would destroy running
+        // threads, which ends the process
+        try {
+            th_.reserve(w);
+            for (int i = 1; i < w; i++) th_.emplace_back([this] { loop(); });
+        } catch (...) {
+        }
     }
     void work() {
         for (;;) {
@@ -719,7 +725,7 @@ int upload_host(Context &C, void *dst, const void *src, size_t bytes) {
         SGPB_CUDA(cudaEventSynchronize(C.stage_ev[slot]));
         try {
             par_copy(buf, (const char *)src + off, n);
-        } catch (...) {   // no threads to be had
+        } catch (...) {   // no memory for the pool
             memcpy(buf, (const char *)src + off, n);
         }
         SGPB_CUDA(cudaMemcpyAsync((char *)dst + off, buf, n, cudaMemcpyHostToDevice, C.stream));
