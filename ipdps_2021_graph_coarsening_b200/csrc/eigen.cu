@@ -1795,12 +1795,13 @@ struct MidLevelDesc {
     const uint32_t *vcmap;
     double *out;             // normalised result (n)
     double *va, *vb, *deg;   // iterate buffers and weighted degrees (n each)
-    uint4 *rows;             // [mid_tiles(m, blocks)][32] rows of each lane's entries (mid_plan)
     double tol;
     uint64_t iter_max;
     double *res;             // [0] niter [1] dot [2] gb [3] lambda [4] capped [6] ms [7] margin (PIArgs)
 };
 
+// The rows of each lane's entries (mid_plan) are a cluster's own: every level
+// that it runs writes them anew.
 // Tiles of kTile entries from the multiple of four at or below a warp's first
 // one: the first tile of the g-th warp of a level, and room for all of them.  A
 // warp of the entries [a, b) has at most (b - a + 130) / kTile of them.
@@ -2015,7 +2016,7 @@ __device__ __forceinline__ void mid_stream(const uint32_t *rp, const uint32_t *c
 
 template <typename W, bool MX, int CL>
 __device__ __forceinline__ void mid_level(const MidLevelDesc &d, cg::cluster_group &cl, double *sm,
-                                          double (*slot)[8]) {
+                                          double (*slot)[8], uint4 *plan) {
     typedef typename std::conditional<MX, float, double>::type ACC;
     const uint32_t n = d.n;
     const uint64_t m = d.m;
@@ -2029,7 +2030,7 @@ __device__ __forceinline__ void mid_level(const MidLevelDesc &d, cg::cluster_gro
     const uint64_t E0 = rp[R0], E1 = rp[R1];
     const uint32_t w0 = wk == 0 ? R0 : rows_at(rp, R0, R1, E0 + (E1 - E0) * wk / kMidWarps);
     const uint32_t w1 = wk + 1 == kMidWarps ? R1 : rows_at(rp, R0, R1, E0 + (E1 - E0) * (wk + 1) / kMidWarps);
-    uint4 *rows = d.rows + mid_tile0(rp[w0], rank * kMidWarps + wk) * 32;
+    uint4 *rows = plan + mid_tile0(rp[w0], rank * kMidWarps + wk) * 32;
     mid_plan(rp, w0, w1, rows);
     // ---- phase 0: start vector (prolongated), weighted degrees, shift
     double p[4] = {0, 0, 0, 0};   // sum x, sum x d, sum d (normlap mean), max d
@@ -2140,8 +2141,9 @@ __device__ __forceinline__ void mid_level(const MidLevelDesc &d, cg::cluster_gro
 template <int CL>
 __global__ void __launch_bounds__(kMidThreads, 1)
     k_power_iter_mid(const MidLevelDesc *__restrict__ lev, const uint2 *__restrict__ chains, uint32_t nchains,
-                     uint32_t *next) {
+                     uint32_t *next, uint4 *plans, uint64_t plan_stride) {
     cg::cluster_group cl = cg::this_cluster();
+    uint4 *plan = plans + (size_t)(blockIdx.x / CL) * plan_stride;
     __shared__ double sm[256];
     __shared__ double slot[2][8];
     __shared__ uint32_t item;
@@ -2161,11 +2163,11 @@ __global__ void __launch_bounds__(kMidThreads, 1)
             const MidLevelDesc &dsc = lev[ch.x + k];
             const unsigned long long t0 = global_ns();
             if (dsc.wbytes == 8) {
-                if (dsc.mixed) mid_level<unsigned long long, true, CL>(dsc, cl, sm, slot);
-                else mid_level<unsigned long long, false, CL>(dsc, cl, sm, slot);
+                if (dsc.mixed) mid_level<unsigned long long, true, CL>(dsc, cl, sm, slot, plan);
+                else mid_level<unsigned long long, false, CL>(dsc, cl, sm, slot, plan);
             } else {
-                if (dsc.mixed) mid_level<uint32_t, true, CL>(dsc, cl, sm, slot);
-                else mid_level<uint32_t, false, CL>(dsc, cl, sm, slot);
+                if (dsc.mixed) mid_level<uint32_t, true, CL>(dsc, cl, sm, slot, plan);
+                else mid_level<uint32_t, false, CL>(dsc, cl, sm, slot, plan);
             }
             // every block's part of the result is written before the next
             // level reads it, and every read of another block's slots is done
@@ -3123,6 +3125,7 @@ bool power_iter_mid_ok(const Level &L, const PowerIterOpts &o) {
 
 int power_iter_mid_chains(Context &C, const std::vector<PIChain *> &chains, const PowerIterOpts &o) {
     const int CLn = o.mid_blocks ? o.mid_blocks : kMidCTAs;   // blocks a cluster
+    uint64_t stride = 0;   // the largest level's row plan
     std::vector<MidLevelDesc> h;
     std::vector<std::pair<uint64_t, uint2>> order;   // (cost, chain) for largest-first
     for (PIChain *ch : chains) {
@@ -3149,7 +3152,8 @@ int power_iter_mid_chains(Context &C, const std::vector<PIChain *> &chains, cons
             SGPB_TRY(dalloc_t(C, &d.va, L.n));
             SGPB_TRY(dalloc_t(C, &d.vb, L.n));
             SGPB_TRY(dalloc_t(C, &d.deg, L.n));
-            SGPB_TRY(dalloc_t(C, &d.rows, mid_tiles(L.m, (uint32_t)CLn) * 32));
+            const uint64_t t = mid_tiles(L.m, (uint32_t)CLn) * 32;
+            stride = t > stride ? t : stride;
             d.tol = o.tol;
             d.iter_max = iter_budget(L.n, o);
             h.push_back(d);
@@ -3197,11 +3201,25 @@ int power_iter_mid_chains(Context &C, const std::vector<PIChain *> &chains, cons
             set_error("the mid-size power-iteration cluster does not fit on the device");
             return SGP_B200_ERR_DEVICE;
         }
-        const uint32_t nclu = (uint32_t)(hc.size() < (size_t)max_clusters ? hc.size() : (size_t)max_clusters);
+        uint32_t nclu = (uint32_t)(hc.size() < (size_t)max_clusters ? hc.size() : (size_t)max_clusters);
+        // a row plan for each cluster; where they do not fit, fewer clusters
+        uint64_t limit = ~0ull;
+        if (const char *e = getenv("SGPB_PI_MID_MB"))   // a limit on the plans
+            if (*e) limit = strtoull(e, nullptr, 10) << 20;
+        uint4 *plans = nullptr;
+        while (true) {
+            C.out_of_memory = false;
+            if (nclu == 1 || nclu * stride * sizeof(uint4) <= limit) {
+                const int rc = dalloc_t(C, &plans, nclu * stride);
+                if (rc == SGP_B200_OK) break;
+                if (nclu == 1 || !C.out_of_memory) return rc;
+            }
+            nclu = (nclu + 1) / 2;
+        }
         cfg.gridDim = dim3(nclu * CL);
         const uint32_t nch = (uint32_t)hc.size();
         SGPB_CUDA(cudaLaunchKernelEx(&cfg, k_power_iter_mid<CL>, (const MidLevelDesc *)lev_d, (const uint2 *)ch_d, nch,
-                                     next));
+                                     next, plans, stride));
         return SGP_B200_OK;
     };
     if (CLn == 2) SGPB_TRY(launch(std::integral_constant<int, 2>()));

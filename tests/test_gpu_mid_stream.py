@@ -8,6 +8,7 @@ Against the oracle after 40 iterations: each rounds the FP64 iterate to about
 import numpy as np
 import pytest
 
+from ipdps_2021_graph_coarsening_b200 import graphs as G
 from oracle import bindings as O
 from tests.test_gpu_slices import csr, dev, weights
 
@@ -56,3 +57,17 @@ def test_mid_stream(partitioner, monkeypatch, name, top, mixed):
     d = np.bincount(np.repeat(np.arange(n), np.diff(rp).astype(np.int64)),
                     None if w is None else w.astype(np.float64), n)
     assert abs(lam - lam_o) <= (1e-5 if mixed else 1e-11) * 4 * d.max()
+
+
+def test_row_plans_of_fewer_clusters(partitioner, monkeypatch):
+    """Row plans that do not fit leave fewer clusters at a time: the batch's
+    results are the same."""
+    gs = G.batch_graphs(24, seed=5, lo=3000, hi=30000)
+    a = partitioner.partition_batch(gs, mixed=True)
+    monkeypatch.setenv("SGPB_PI_MID_MB", "1")
+    b = partitioner.partition_batch(gs, mixed=True)
+    monkeypatch.setenv("SGPB_PI_MID_MB", "0")
+    c = partitioner.partition_batch(gs, mixed=True)
+    for x, y, z in zip(a, b, c):
+        assert np.array_equal(x.part, y.part) and np.array_equal(x.part, z.part)
+        assert x.lam == y.lam == z.lam and x.level_iters == y.level_iters == z.level_iters
