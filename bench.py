@@ -129,6 +129,18 @@ def algorithmic_pi_bytes(n: int, m: int, weighted: bool, s: int) -> int:
     return 4 * (n + 1) + 4 * m + (4 * m if weighted else 0) + s * n + s * n + 4 * n
 
 
+def layout_pi_bytes(n: int, m: int, finest: bool) -> int:
+    """Bytes an iteration streams at least, by the layout of the kernel that runs
+    the level: the finest level's CSR (4-byte destinations and offsets), row
+    slices elsewhere (2-byte destinations, weights not counted, a sum per row and
+    panel of 25,600 columns written and read), the iterate read and written,
+    the degrees."""
+    if finest:
+        return algorithmic_pi_bytes(n, m, False, 8)
+    panels = -(-n // 25600)
+    return 2 * m + 3 * 8 * n + (2 * 8 * panels * n if panels > 1 else 0)
+
+
 def algorithmic_coarsen_bytes(level_n, level_m, level_rounds, wbytes: int = 4) -> int:
     """Bytes the coarsening of a hierarchy must move (the per-level model):
     the heavy-neighbour scan 4(n+1) + 4m + w*m (weighted levels) + 4n, the map
@@ -366,22 +378,22 @@ def gpu_arm(args, rank: int, ws: int, local: int, distmod):
     if ws == 1 and not args.no_batch:
         batch = batch_leg(p, value)
 
-    # roofline of the dominant kernel (power iteration) from this step's levels
+    # roofline of the dominant kernel (power iteration) from this step's levels:
+    # the bytes its layouts stream, and beside them the rate of a kernel that
+    # reads 8 bytes an entry (CSR with 4-byte weights) and takes the same time
     peak, peak_kind = load_peaks()
-    byts = sum(it * algorithmic_pi_bytes(nl, ml, l > 0, 8)
-               for l, (nl, ml, it) in enumerate(zip(r.level_n, r.level_m, r.level_iters)))
+    levels = list(enumerate(zip(r.level_n, r.level_m, r.level_iters)))
+    byts = sum(it * layout_pi_bytes(nl, ml, l == 0) for l, (nl, ml, it) in levels)
+    byts_csr = sum(it * algorithmic_pi_bytes(nl, ml, l > 0, 8) for l, (nl, ml, it) in levels)
     pi_ms = sum(r.level_pi_ms)
     achieved = byts / (pi_ms / 1e3) / 1e9 if pi_ms > 0 else 0.0
-    # DRAM bytes (read + write) of the step's power-iteration launches: the
-    # ratio of measured DRAM bytes to algorithmic bytes from one ncu capture of
-    # the CSR kernel on a smaller level, applied to this step's algorithmic
-    # bytes: an upper bound for row slices, which read about 2.2 bytes an entry
-    # of the largest coarse level where the model counts 8
+    # DRAM bytes (read + write): the ratio of measured to layout bytes from one
+    # ncu capture of this graph's largest coarse level, applied to the step
     traffic = None
     tf = os.path.join(ROOT, "profiles", "power_iter_traffic.json")
     if os.path.exists(tf):
         try:
-            ratio = json.load(open(tf)).get("dram_to_algorithmic_ratio")
+            ratio = json.load(open(tf)).get("dram_to_layout_ratio")
             traffic = ratio * byts if ratio else None
         except (OSError, ValueError):
             traffic = None
@@ -395,7 +407,8 @@ def gpu_arm(args, rank: int, ws: int, local: int, distmod):
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": traffic, "kernel": "k_pi_slices (+ k_power_iter on the finest level, k_power_iter_chains on the small levels)",
                 "peak_kind": peak_kind,
-                "kernel_ms_per_step": pi_ms, "algorithmic_bytes_per_step": byts,
+                "kernel_ms_per_step": pi_ms, "layout_bytes_per_step": byts,
+                "csr_model_gbs": byts_csr / (pi_ms / 1e3) / 1e9 if pi_ms > 0 else 0.0,
                 "kernel_share_of_step": pi_ms / ms if ms else None}
 
     line = {"metric": METRIC, "value": value, "unit": "edges/s", "n_gpus": ws, "steps": args.steps,
