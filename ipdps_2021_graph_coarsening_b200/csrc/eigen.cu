@@ -1682,7 +1682,8 @@ __device__ __noinline__ void small_level_rows(const PIArgs &a) {
             dot = s_ur * inv_n;
             niter++;
             const double delta = fabs(dot - last);
-            margin = nsq > r_min ? fmin(margin, fabs(delta - a.tol)) : 0.0;
+            // (one warp: with all 32 an iteration takes 0.07 us more)
+            if (wid == 0) margin = nsq > r_min ? fmin(margin, fabs(delta - a.tol)) : 0.0;
             if (!(delta > a.tol && niter < a.iter_max)) break;
             mu = mu_n;
             inv_nu = inv_n;
@@ -2118,7 +2119,7 @@ __device__ __forceinline__ void mid_level(const MidLevelDesc &d, cg::cluster_gro
         dot = (P[2] - mu_n * P[3]) * inv_nu_n;
         niter++;
         const double delta = fabs(dot - last);
-        margin = nsq > kCancel * gb * gb ? fmin(margin, fabs(delta - d.tol)) : 0.0;
+        if (wk == 0) margin = nsq > kCancel * gb * gb ? fmin(margin, fabs(delta - d.tol)) : 0.0;
         if (!(delta > d.tol && niter < d.iter_max)) {
             for (uint32_t i = R0 + threadIdx.x; i < R1; i += blockDim.x) d.out[i] = (src[i] - mu) * inv_nu;
             if (rank == 0 && threadIdx.x == 0) {
