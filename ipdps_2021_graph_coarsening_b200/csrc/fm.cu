@@ -26,6 +26,8 @@
 // Passes repeat until one applies nothing or leaves the cut unchanged.
 #include <cooperative_groups.h>
 
+#include <stdlib.h>
+
 #include <type_traits>
 
 #include "bits.cuh"
@@ -135,8 +137,11 @@ __global__ void k_fm_list(uint32_t n2, const uint32_t *__restrict__ flag, const 
 }
 
 // Counting sort of both sides' candidates (the first na of the list are side
-// 0's): key = side, then the descending bucket.
+// 0's): key = side, then the descending bucket.  Above kFmJoint candidates a side
+// at a time (half the keys, na = len), so that keys times tiles fit 32 bits and
+// the histogram stays at 8 bytes a candidate.
 constexpr int kFmKeys = 2 * kFmBuckets;
+constexpr uint64_t kFmJoint = 1ull << 28;
 __device__ __forceinline__ uint32_t fm_key(uint32_t i, uint32_t na, long long g) {
     return (i < na ? 0u : (uint32_t)kFmBuckets) + (uint32_t)(kFmBuckets - 1) - fm_bucket(g);
 }
@@ -144,24 +149,24 @@ __device__ __forceinline__ uint32_t fm_key(uint32_t i, uint32_t na, long long g)
 // counts per (key, tile): hist[key * ntiles + t]
 __global__ void __launch_bounds__(kFmTile) k_fm_hist(uint32_t len, uint32_t na, const uint32_t *__restrict__ idx,
                                                      const long long *__restrict__ gain, uint32_t ntiles,
-                                                     uint32_t *__restrict__ hist) {
+                                                     int keys, uint32_t *__restrict__ hist) {
     __shared__ uint32_t cnt[kFmKeys];
-    for (int b = threadIdx.x; b < kFmKeys; b += blockDim.x) cnt[b] = 0;
+    for (int b = threadIdx.x; b < keys; b += blockDim.x) cnt[b] = 0;
     __syncthreads();
     const uint32_t i = blockIdx.x * kFmTile + threadIdx.x;
     if (i < len) atomicAdd(&cnt[fm_key(i, na, gain[idx[i]])], 1u);
     __syncthreads();
-    for (int b = threadIdx.x; b < kFmKeys; b += blockDim.x) hist[(size_t)b * ntiles + blockIdx.x] = cnt[b];
+    for (int b = threadIdx.x; b < keys; b += blockDim.x) hist[(size_t)b * ntiles + blockIdx.x] = cnt[b];
 }
 
 // stable placement: within a tile the warps take turns in order, and lanes
 // of one key rank by lane
 __global__ void __launch_bounds__(kFmTile) k_fm_place(uint32_t len, uint32_t na, const uint32_t *__restrict__ idx,
                                                       const long long *__restrict__ gain, uint32_t ntiles,
-                                                      const uint32_t *__restrict__ off,
+                                                      int keys, const uint32_t *__restrict__ off,
                                                       uint32_t *__restrict__ sorted) {
     __shared__ uint32_t cnt[kFmKeys];
-    for (int b = threadIdx.x; b < kFmKeys; b += blockDim.x) cnt[b] = 0;
+    for (int b = threadIdx.x; b < keys; b += blockDim.x) cnt[b] = 0;
     __syncthreads();
     const uint32_t i = blockIdx.x * kFmTile + threadIdx.x;
     const bool valid = i < len;
@@ -388,12 +393,36 @@ static int fm_impl(Context &C, const Level &L, const W *w, uint32_t *part, uint3
     SGPB_TRY(dalloc_t(C, &pos, 2 * (size_t)n + 1));
     SGPB_TRY(dalloc_t(C, &side, n));
     SGPB_TRY(dalloc_t(C, &idx, n));
-    SGPB_TRY(dalloc_t(C, &sorted, n));
-    SGPB_TRY(dalloc_t(C, &order, n));
-    SGPB_TRY(dalloc_t(C, &rank, n));
+    // once the candidates are listed, flags and positions have been read
+    sorted = pos;
+    order = flag;
+    rank = flag + n;
     SGPB_TRY(dalloc_t(C, &sums, 4));
     SGPB_TRY(dalloc_t(C, &best, 1));
-    uint32_t hist_tiles = 0;   // tiles hist and off have room for
+    size_t hist_room = 0;   // entries of hist and off
+    uint64_t joint = kFmJoint;
+    if (const char *e = getenv("SGPB_FM_JOINT"))   // another bound (0: always a side at a time)
+        if (*e) joint = strtoull(e, nullptr, 10);
+    // len candidates (the first na are side 0's) of src in order into dst
+    auto sort = [&](uint32_t len, uint32_t na, const uint32_t *src, uint32_t *dst, int keys) -> int {
+        if (!len) return SGP_B200_OK;
+        const uint32_t nt = cdiv(len, kFmTile);
+        const uint64_t cells = (uint64_t)keys * nt;
+        if (cells > 0xFFFFFFFFull) {
+            set_error("FM: %u candidates of one side", len);
+            return SGP_B200_ERR_TOO_LARGE;
+        }
+        if (cells > hist_room) {
+            SGPB_TRY(dalloc_t(C, &hist, cells + 1));
+            SGPB_TRY(dalloc_t(C, &off, cells + 1));
+            hist_room = cells;
+        }
+        k_fm_hist<<<nt, kFmTile, 0, C.stream>>>(len, na, src, gain, nt, keys, hist);
+        SGPB_TRY(scan_u32(C, hist, off, (uint32_t)cells, nullptr));
+        k_fm_place<<<nt, kFmTile, 0, C.stream>>>(len, na, src, gain, nt, keys, off, dst);
+        C.kernel_launches += 2;
+        return SGP_B200_OK;
+    };
     int per_sm = 0;
     SGPB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fm_best, 256, 0));
     if (per_sm < 1) {
@@ -472,20 +501,13 @@ static int fm_impl(Context &C, const Level &L, const W *w, uint32_t *part, uint3
                 k_fm_list<<<cdiv(n, 256), 256, 0, C.stream>>>(n, flag + (size_t)sd * n, pos, n, idx + (sd ? na : 0));
             }
         }
-        const uint32_t nt = cdiv(k, kFmTile);
-        if ((uint64_t)kFmKeys * nt > 0xFFFFFFFFull) {
-            set_error("FM: %u vertices of positive gain; their sort holds fewer than 2^31", k);
-            return SGP_B200_ERR_TOO_LARGE;
+        C.kernel_launches += 1;
+        if (k <= joint) {
+            SGPB_TRY(sort(k, na, idx, sorted, kFmKeys));
+        } else {
+            SGPB_TRY(sort(na, na, idx, sorted, kFmBuckets));
+            SGPB_TRY(sort(nb, nb, idx + na, sorted + na, kFmBuckets));
         }
-        if (nt > hist_tiles) {
-            SGPB_TRY(dalloc_t(C, &hist, (size_t)kFmKeys * nt + 1));
-            SGPB_TRY(dalloc_t(C, &off, (size_t)kFmKeys * nt + 1));
-            hist_tiles = nt;
-        }
-        k_fm_hist<<<nt, kFmTile, 0, C.stream>>>(k, na, idx, gain, nt, hist);
-        SGPB_TRY(scan_u32(C, hist, off, kFmKeys * nt, nullptr));
-        k_fm_place<<<nt, kFmTile, 0, C.stream>>>(k, na, idx, gain, nt, off, sorted);
-        C.kernel_launches += 3;
         const uint32_t *sa = sorted, *sb = sorted + na;
         const unsigned long long key0 = ((unsigned long long)cut0 << 32) | 0xFFFFFFFFull;
         SGPB_TRY(dzero(C, listed, sizeof(uint32_t) * words));   // ranks are read of listed vertices alone

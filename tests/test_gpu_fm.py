@@ -55,3 +55,18 @@ def test_partition_with_fm(partitioner, name):
     # the same passes from the same split on the oracle
     op, oc, _, _ = O.fm_refine(g.row_ptr, g.col, None, base.part, 16)
     assert np.array_equal(r.part, op) and r.edgecut == oc
+
+
+@pytest.mark.parametrize("name", ["er", "rmat"])
+def test_candidates_of_a_side_at_a_time(partitioner, monkeypatch, name):
+    """The candidate sort of calls too large for both sides at once."""
+    monkeypatch.setenv("SGPB_FM_JOINT", "0")
+    g = CASES[name]()
+    rp = torch.from_numpy(g.row_ptr.view(np.int32)).cuda()
+    col = torch.from_numpy(g.col.view(np.int32)).cuda()
+    for label, p0 in starts(g).items():
+        pd = torch.from_numpy(p0.astype(np.uint32).view(np.int32)).cuda()
+        cut, passes, moves = partitioner.fm_refine(rp, col, pd, 16)
+        op, oc, opasses, omoves = O.fm_refine(g.row_ptr, g.col, None, p0, 16)
+        assert (passes, moves, cut) == (opasses, omoves, oc), label
+        assert np.array_equal(pd.cpu().numpy().view(np.uint32), op), label
