@@ -238,9 +238,8 @@ def batch_graphs_cached():
     cache = os.path.join("/tmp", "sgpb_batch2048.npz")
     if os.path.exists(cache):
         d = np.load(cache)
-        off_r, off_c = d["off_r"], d["off_c"]
-        return [G.CSR(d["rp"][off_r[i]:off_r[i + 1]], d["col"][off_c[i]:off_c[i + 1]])
-                for i in range(len(off_r) - 1)]
+        off_r, off_c, rp, col = d["off_r"], d["off_c"], d["rp"], d["col"]   # an npz reads a member on every access
+        return [G.CSR(rp[off_r[i]:off_r[i + 1]], col[off_c[i]:off_c[i + 1]]) for i in range(len(off_r) - 1)]
     gs = G.batch_graphs(2048)
     try:
         off_r = np.cumsum([0] + [g.n + 1 for g in gs])
