@@ -603,10 +603,12 @@ __global__ void __launch_bounds__(WARPS * 32) k_dedupe_bits(const uint32_t *__re
     }
 }
 
-// threads of the bitmap's blocks that have to fit an SM.  R-MAT 22's builds:
-// 12.1 ms with the radix sort alone, 10.35 at 256, 10.05 at 384, 10.35 at 512
-// (its first build has 284,257 destinations, where the blocks of 64 threads
-// leave at 384 and those of 128 at 512)
+// threads of the bitmap's blocks that have to fit an SM.  Builds of whole
+// hierarchies with the radix sort alone / 256 / 384 / 512 / whenever one fits, ms:
+// R-MAT 22 12.0 / 10.1 / 9.9 / 10.4 / 10.2, R-MAT 20 3.65 / 2.89 / 2.90 / 2.90 /
+// 2.90, weighted Chung-Lu of 1,200,001 vertices 7.31 / 6.13 / 6.10 / 6.12 / 7.30,
+// Erdos-Renyi of 500,003 vertices of 40 entries 3.73 / 2.89 / 2.89 / 3.03 / 2.87,
+// of 1,000,003 of 8 2.71 / 2.13 / 2.13 / 2.15 / 2.28
 constexpr uint32_t kBitsMinThreads = 384;
 
 // The tier's kernel for a level of nc coarse vertices: the bitmap where

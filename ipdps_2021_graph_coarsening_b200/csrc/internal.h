@@ -242,6 +242,7 @@ struct PIChainLevel {
 struct PIChain {
     const double *x0 = nullptr;
     std::vector<PIChainLevel> lev;
+    bool plain = false;   // in the plain order of sums, whatever the launch's options
 };
 int power_iter_chains(Context &C, const std::vector<PIChain *> &chains, const PowerIterOpts &o);
 // Mid-size levels (a cluster of blocks, the iterate in global memory, one

@@ -706,7 +706,7 @@ static int upload_text(Context &C, MtxSource &src, uint8_t *dtext) {
 // A host array to the device: pinned and small arrays in one copy, large
 // pageable ones through the pinned ring.  The runtime stages pageable memory
 // on one thread, about 11 GB/s: the coarsening call on R-MAT 20 (122 MB of
-// destinations) 16.3 -> 7.9 ms, of R-MAT 19 9.2 -> 5.4, R-MAT 18 4.7 -> 4.0.
+// destinations) 17.5 -> 9.3 ms.
 int upload_host(Context &C, void *dst, const void *src, size_t bytes) {
     const size_t chunk = stage_slot(bytes, kUploadSlotBytes);
     bool ring = bytes >= kUploadMin && is_pageable(src);

@@ -327,7 +327,7 @@ static int launch_cut_bits(cudaStream_t s, int num_sms, uint32_t n, const uint32
                            unsigned long long *out) {
     const uint32_t words = bit_words(n);
     const size_t bytes = (size_t)words * 4;
-    // two blocks an SM while two bitmaps fit; a block per 4096 rows at least
+    // two blocks an SM while two bitmaps fit, of at least 256 rows each
     uint32_t g = (uint32_t)num_sms * (words <= kBitsMaxWords / 2 || words > kBitsMaxWords ? 2u : 1u);
     if (g > cdiv(n, 256)) g = cdiv(n, 256);
     if (words <= kBitsMaxWords) {

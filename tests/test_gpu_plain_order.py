@@ -72,6 +72,16 @@ def test_batch_and_4way_are_the_plain_order_s(partitioner, monkeypatch):
             assert np.array_equal(a[0], b[0]) and a[1:] == b[1:]
 
 
+def test_a_batch_of_both_kinds(partitioner, monkeypatch):
+    """Graphs that start in the plain order (mostly leaves) beside ones that do
+    not, of which some are repeated; waves of one kind first and last."""
+    gs = [make(s) for make, seeds in GRAPHS for s in seeds]
+    grids = [G.grid2d(200, 150), G.grid2d(40, 30), G.erdos_renyi(40000, 8.0, seed=2), G.rmat(12, seed=3)]
+    for batch in (grids + gs, gs, gs[:3] + grids[1:2]):
+        for a, b in zip(*both(monkeypatch, lambda: partitioner.partition_batch(batch, rng_state=1007))):
+            same(a, b)
+
+
 @pytest.mark.parametrize("n", [700, 20000])   # one block's rows form, row slices
 def test_a_stop_within_rounding_of_the_tolerance(partitioner, monkeypatch, n):
     g = G.erdos_renyi(n, 8.0, seed=3)
