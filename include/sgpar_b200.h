@@ -156,7 +156,10 @@ typedef struct {
                                    sum_j w_ij (x_i - x_j) with FP32 differences,
                                    products and row sums; the iterate, shift,
                                    deflation, normalisation, dot product and
-                                   stopping test stay FP64 */
+                                   stopping test stay FP64.  Slower than FP64 on one
+                                   large graph (R-MAT 22: 197 against 81 ms), whose
+                                   FP64 levels run on row slices; faster in
+                                   sgp_b200_partition_batch */
     int perc_imbalance;         /* sgp_compute_partition's perc_imbalance_allowed */
     uint64_t iter_cap;          /* extra cap on power iterations per level, 0 = none */
     uint64_t rng_state, rng_inc;/* PCG32 seeding (advanced copy returned in result) */
