@@ -1029,7 +1029,9 @@ int sgp_b200_power_iter(sgp_b200_ctx_t *x, uint32_t n, const uint32_t *rp, const
     o.tol = tol;
     o.iter_cap = iter_cap;
     o.mixed = mixed;
-    o.plain = x_in == x_out;   // the result may be needed in the other order, from the same vector
+    // the level may be needed once more from the same vector (close): a result
+    // written over it leaves the plain order alone
+    o.plain = x_in < x_out + n && x_out < x_in + n;
     PowerIterResult r;
     if (rc == SGP_B200_OK) rc = power_iter_level(*C, L, x_in, vcmap, x_out, o, &r, residual != nullptr);
     if (rc == SGP_B200_OK && r.close) {

@@ -7,9 +7,12 @@ repeated in the plain order where the certificate fails: the median among
 values that are equal in exact arithmetic (leaves of one aggregate), an
 iteration that stops within rounding of the tolerance, an iterate that
 cancels.  Bit for bit against the plain order."""
+import ctypes
+
 import numpy as np
 import pytest
 
+from ipdps_2021_graph_coarsening_b200 import _lib as L
 from ipdps_2021_graph_coarsening_b200 import graphs as G
 from tests.test_gpu_parity import dev_u32
 
@@ -122,3 +125,23 @@ def test_a_few_iterations_do_without_the_layout(partitioner, monkeypatch, n):
     x = torch.from_numpy(np.random.default_rng(2).random(g.n)).cuda()
     a, b = both(monkeypatch, lambda: partitioner.power_iter(rp, col, None, x, iter_cap=4, residual=False))
     assert a[1] == b[1] == 4 and torch.equal(a[0], b[0])
+
+
+@pytest.mark.parametrize("at", [-5, 0, 5])
+def test_a_result_over_the_start_vector(partitioner, monkeypatch, at):
+    """x_out may lie over x_in, which is read before the first iteration."""
+    g = G.erdos_renyi(20000, 8.0, seed=6)
+    rp, col = dev_u32(g.row_ptr), dev_u32(g.col)
+    x = np.random.default_rng(3).random(g.n)
+    monkeypatch.setenv("SGPB_PI_SLICES", "0")
+    want = partitioner.power_iter(rp, col, None, torch.from_numpy(x).cuda(), residual=False)
+    monkeypatch.delenv("SGPB_PI_SLICES")
+    buf = torch.zeros(g.n + 10, dtype=torch.float64, device="cuda")
+    buf[5:5 + g.n] = torch.from_numpy(x).cuda()
+    torch.cuda.synchronize()
+    iters, lam = ctypes.c_uint64(0), ctypes.c_double(0)
+    ptr = buf.data_ptr() + 40
+    L.check(L.lib().sgp_b200_power_iter(partitioner._ctx, g.n, rp.data_ptr(), col.data_ptr(), None, 0, ptr, None,
+                                        ptr + 8 * at, 1e-10, 0, 0, ctypes.byref(iters), ctypes.byref(lam), None),
+            "sgp_b200_power_iter")
+    assert iters.value == want[1] and torch.equal(buf[5 + at:5 + at + g.n], want[0])
