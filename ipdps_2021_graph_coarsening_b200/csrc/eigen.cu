@@ -1481,8 +1481,8 @@ __device__ __forceinline__ void small_level(const PIArgs &a) {
 // and combined by every warp for itself, so an iteration has one barrier.  The
 // fifth sum (u.u, for the eigenvalue) is taken once, at the end.  What is left
 // is the chain of a gather (65 clocks), the sums' shuffles (218 for the three)
-// and the reciprocal root (78).  24 vertices: 2.29 -> 0.63 us an iteration, 239
-// vertices 2.43 -> 1.25, 773 vertices 3.34 -> 1.94, 528 vertices of 13 entries a
+// and the reciprocal root (78).  24 vertices: 2.29 -> 0.67 us an iteration, 239
+// vertices 2.43 -> 1.26, 773 vertices 3.34 -> 1.98, 528 vertices of 13 entries a
 // row 11.8 -> 3.4.
 constexpr int kHeld = 8;
 

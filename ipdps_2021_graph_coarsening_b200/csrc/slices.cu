@@ -8,7 +8,8 @@
 // entries; rows above 32 * epl entries are cut into units of that size.  Rows
 // are summed by their lanes in entry order and combined by a butterfly.
 //
-// Four forms, chosen per level (slice_form):
+// Four forms, chosen per level (slice_form; the direct ones take a second
+// barrier where a row is far above a block's share, kLongRowGlobal):
 //   direct, shared   the whole iterate in every block's shared memory
 //                    (n <= kSlicePW), one grid barrier an iteration
 //   panels           columns cut into panels of kSlicePW; a block loads the
