@@ -157,9 +157,9 @@ typedef struct {
                                    products and row sums; the iterate, shift,
                                    deflation, normalisation, dot product and
                                    stopping test stay FP64.  Slower than FP64 on one
-                                   large graph (R-MAT 22: 197 against 81 ms), whose
-                                   FP64 levels run on row slices; faster in
-                                   sgp_b200_partition_batch */
+                                   large graph (R-MAT 22: 195 against 82 ms), whose
+                                   FP64 levels run on row slices; a few per cent
+                                   faster in sgp_b200_partition_batch */
     int perc_imbalance;         /* sgp_compute_partition's perc_imbalance_allowed */
     uint64_t iter_cap;          /* extra cap on power iterations per level, 0 = none */
     uint64_t rng_state, rng_inc;/* PCG32 seeding (advanced copy returned in result) */
